@@ -174,17 +174,14 @@ uint16_t par2cuda_coeff(uint16_t input_num, uint16_t exponent);
  * rows).  Returns the previous setting. */
 int par2cuda_set_comb_shape(int shape);
 /* Tile shape of the block-scaled 4-bit tensor method for every later call in
- * this process (the autotuner's knob): 0 = chosen from the number of inputs,
- * 1 = 128 words x 16 recovery slices with one TMEM accumulator, 2 = 128 words
- * x 12 recovery slices with two accumulators (a tile's read-out overlaps the
- * next tile's MMAs).  Returns the previous setting.  No counterpart in the
- * reference. */
+ * this process (the autotuner's knob): 0 = automatic, 1 = up to 240 columns
+ * per tile, 2 = up to 128.  Returns the previous setting.  No counterpart in
+ * the reference. */
 int par2cuda_set_tc4_shape(int shape);
 /* Raster group of the tensor_fp4 GEMM for every later call in this process
- * (the autotuner's knob): the number of 128-word tiles that walk the recovery
- * tiles together; 0 = chosen from the input count (as many as keep their
- * expanded input planes in about 48 MiB of L2).  Returns the previous
- * setting.  No counterpart in the reference. */
+ * (the autotuner's knob): the number of 256-word tiles that walk the column
+ * tiles together; 0 = automatic.  Returns the previous setting.  No
+ * counterpart in the reference. */
 int par2cuda_set_tc4_group(int word_tiles);
 /* The tile shape (1 or 2) the next tensor_fp4 call with num_in inputs will use. */
 int par2cuda_tc4_shape_for(unsigned num_in);
@@ -223,9 +220,9 @@ size_t par2cuda_muladd_scratch_bytes(unsigned num_rec, unsigned num_in);
  * tile).  No counterpart in the reference. */
 size_t par2cuda_tensor_fp4_scratch_bytes(unsigned num_rec, unsigned num_in, size_t n_words);
 /* Measures the tensor pipe's rate (binary multiply-accumulates per second)
- * for the MMA of PAR2CUDA_METHOD_TENSOR_FP4 (M=128, N=256, K=64, mxf4) with one
- * CTA per SM issuing MMAs on shared-memory operands (about 0.1 s): the
- * roofline denominator of that method.  No counterpart in the reference. */
+ * for the MMA of PAR2CUDA_METHOD_TENSOR_FP4 (a CTA pair's M=256, N=240, K=96,
+ * mxf4) issued on shared-memory operands (about 0.1 s): the roofline
+ * denominator of that method.  No counterpart in the reference. */
 int par2cuda_tensor_fp4_rate(double* macs_per_s, void* stream);
 /* The number of kernel launches one par2cuda_muladd call with these
  * arguments makes (the tensor_fp4 method: one per word chunk of expanded

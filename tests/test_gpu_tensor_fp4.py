@@ -82,3 +82,70 @@ def test_fp4_accumulate_and_word_chunks(shape):
     got, want = run_fp4(n, R, S, seed=5, accumulate=True, scratch_bytes=small, shape=shape)
     assert np.array_equal(got, want)
     assert L.par2cuda_tensor_fp4_scratch_bytes(R, n, S // 2) >= small
+
+
+@pytest.mark.parametrize("n,R,words,acc", [
+    (960, 240, 19456, False),    # two whole stages of units, one full column tile, one tile per CTA pair
+    (961, 472, 19301, True),     # a unit with one input, two column tiles, the last pair's second half past the words
+    (1437, 240, 38000, False),   # three stages, two tiles per pair
+    (2000, 200, 19455, True),    # a last stage of one unit, a tile that is not full
+    (4096, 480, 9728, False),    # long passes
+])
+def test_fp4_long_passes_match_the_table_kernel(n, R, words, acc):
+    # sizes at which single-bit passes over full column tiles are chosen,
+    # against the table kernel (itself compared with the oracle)
+    import torch
+    L = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(n + R)
+    pw = (words + 63) // 64 * 64
+    d_in, d_rec, d_coeff = (torch.randint(-32768, 32768, shape, generator=g, device="cuda").to(torch.int16)
+                            for shape in ((n, pw), (R, pw), (R, n)))
+    got = {}
+    for method in (_lib.METHOD_COMB, _lib.METHOD_TENSOR_FP4):
+        rec = d_rec.clone()
+        sb = L.par2cuda_muladd_scratch_bytes(R, n)
+        if method == _lib.METHOD_TENSOR_FP4:
+            sb = L.par2cuda_tensor_fp4_scratch_bytes(R, n, words)
+        scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+        assert L.par2cuda_muladd(d_in.data_ptr(), pw, n, d_coeff.data_ptr(), rec.data_ptr(), pw, R, words, int(acc), method,
+                                 scratch.data_ptr(), sb, None) == 0, L.par2cuda_last_error()
+        torch.cuda.synchronize()
+        got[method] = rec
+    assert L.par2cuda_device_error() == 0
+    assert torch.equal(got[_lib.METHOD_COMB][:, :words], got[_lib.METHOD_TENSOR_FP4][:, :words])
+    # nothing past the words was written
+    assert torch.equal(got[_lib.METHOD_TENSOR_FP4][:, words:], d_rec[:, words:])
+
+
+@pytest.mark.parametrize("n,R,S", [(96, 240, 512), (97, 241, 514), (480, 224, 2050), (577, 500, 1030)])
+def test_fp4_many_recovery_slices(n, R, S):
+    got, want = run_fp4(n, R, S, seed=n + 7 * R)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("n,R,S", [(24, 60, 512), (25, 61, 510), (121, 4, 130000), (600, 120, 66000)])
+def test_fp4_few_recovery_slices(n, R, S):
+    # tile and unit edges of the form of four bits per pass; many tiles per CTA pair
+    got, want = run_fp4(n, R, S, seed=3 * n + R, accumulate=True)
+    assert np.array_equal(got, want)
+
+
+def test_fp4_forms_agree_with_the_field():
+    # every coefficient bit against every word bit: 16 x 16 single-bit products
+    import torch
+    L = _lib.load()
+    n, R, nw = 16, 16, 256
+    words = np.zeros((n, nw), dtype=np.uint16)
+    for b in range(16):
+        words[b, b * 16:(b + 1) * 16] = 1 << np.arange(16, dtype=np.uint32)
+    coeff = np.array([[1 << ((r + i) % 16) for i in range(n)] for r in range(R)], dtype=np.uint16)
+    d_in = torch.from_numpy(words.view(np.int16)).cuda()
+    d_coeff = torch.from_numpy(coeff.view(np.int16)).cuda()
+    d_rec = torch.zeros((R, nw), dtype=torch.int16, device="cuda")
+    sb = L.par2cuda_tensor_fp4_scratch_bytes(R, n, nw)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+    assert L.par2cuda_muladd(d_in.data_ptr(), nw, n, d_coeff.data_ptr(), d_rec.data_ptr(), nw, R, nw, 0,
+                             _lib.METHOD_TENSOR_FP4, scratch.data_ptr(), sb, None) == 0
+    torch.cuda.synchronize()
+    want = O.recover_coeffs(words.view(np.uint8), np.full(n, 2 * nw), coeff).view(np.int16)
+    assert np.array_equal(d_rec.cpu().numpy(), want)
