@@ -9,12 +9,18 @@
 // MD5 is RFC 1321; CRC32 is the reflected IEEE polynomial 0xEDB88320.  The
 // zero padding of the CRC is applied by multiplying the register by
 // x^(8*pad) mod P (hasher/crc_zeropad.c:55-66); the MD5 must process the
-// padding bytes.  The CRC is computed slice-by-4 from shared-memory tables in
-// the same thread, in the bubbles of the MD5 dependency chain.
+// padding bytes.  The CRC is computed from shared-memory tables by other warps
+// of the block, beside the MD5 chains.
 #include "common.cuh"
 #include "kernels.h"
 
 namespace p2c {
+
+// chains per warp of the hash kernels with a block of many rows or files: the
+// loads of 32 chains of a warp are 32 separate lines or rows of banks, and
+// delay each other; one thread hashes 127.6 MB/s among 32 of a warp, 130.5
+// among 16 and 135.0 among 8 (two warps a scheduler for 64 chains)
+#define P2C_MD5_LANES 8
 
 // RFC 1321 round constants (a constexpr table: indexed by the unrolled step
 // number, each becomes an immediate operand).
@@ -55,83 +61,126 @@ __device__ __forceinline__ void md5_block(uint32_t st[4], const uint32_t m[16]) 
 	st[0] += a; st[1] += b; st[2] += c; st[3] += d;
 }
 
-struct CrcTabs;
-__device__ __forceinline__ uint32_t crc_word(const CrcTabs& T, uint32_t crc, uint32_t w);
-struct NoTabs {};
-__device__ __forceinline__ uint32_t crc_word(const NoTabs&, uint32_t crc, uint32_t) { return crc; }
-
-__device__ __forceinline__ void load_block(const uint4* p4, size_t b, uint32_t m[16]) {
+struct MsgBlock {
+	uint32_t w[16];
+	__device__ __forceinline__ explicit MsgBlock(const uint32_t (&m)[16]) {
 #pragma unroll
-	for(int q = 0; q < 4; q++) {
-		uint4 v = __ldg(p4 + b * 4 + q);
-		m[4 * q] = v.x; m[4 * q + 1] = v.y; m[4 * q + 2] = v.z; m[4 * q + 3] = v.w;
+		for(int q = 0; q < 16; q++) w[q] = m[q];
 	}
-}
+};
 
-// MD5 (and optionally CRC32) over `full` consecutive 64-byte blocks with the
-// loads software-pipelined two blocks ahead: a single thread walks a long
-// serial chain, so without prefetch every block would wait a full memory
-// latency.
+// MD5 over `full` consecutive 64-byte blocks whose first word p lies C words
+// (0..3) before a 16-byte boundary.  A single thread walks a long serial
+// chain, so loads run two blocks ahead of it; each block's words stay where
+// they were loaded (C > 0: the last C words of the load before it and the
+// first 16 - C of its own), in three (four) buffers that the unrolled loop
+// takes in turn, because copies and loads gathered between two blocks delay
+// the chain: one thread hashes 144 MB/s this way and 138 with a copy per
+// block (C = 0; 120 with a copy for C > 0).
 // L2 prefetch distance (64-byte blocks) ahead of the register prefetch: the
 // register loads then mostly hit L2, well inside their two-block lead
 #define P2C_MD5_L2_AHEAD 48
 
-template<bool CRC, typename Tabs>
-__device__ __forceinline__ void md5_blocks(uint32_t st[4], uint32_t& crc, const Tabs& T, const uint4* p4, size_t full) {
-	uint32_t A[16], B[16];
-	if(full > 0) load_block(p4, 0, A);
-	if(full > 1) load_block(p4, 1, B);
-	for(size_t b = 0; b < full; b += 2) {
-		uint32_t m[16];
-		// one 128-byte line (two blocks) per iteration, only inside this row
-		if(b + P2C_MD5_L2_AHEAD < full)
-			asm volatile("prefetch.global.L2 [%0];" :: "l"(p4 + (b + P2C_MD5_L2_AHEAD) * 4));
+// load k holds words C + 16 k ..; words the blocks do not need (the last C of
+// the last load) are not read
+template<int C>
+__device__ __forceinline__ void md5_load(const uint32_t* p, size_t k, bool last, uint32_t (&m)[16]) {
+	const uint4* p4 = reinterpret_cast<const uint4*>(p + C) + k * 4;
 #pragma unroll
-		for(int q = 0; q < 16; q++) m[q] = A[q];
-		if(b + 2 < full) load_block(p4, b + 2, A);
-		if(CRC) {
+	for(int q = 0; q < 4; q++) {
+		if(C == 0 || q < 3 || !last) {
+			const uint4 v = __ldg(p4 + q);
+			m[4 * q] = v.x; m[4 * q + 1] = v.y; m[4 * q + 2] = v.z; m[4 * q + 3] = v.w;
+		} else {
 #pragma unroll
-			for(int q = 0; q < 16; q++) crc = crc_word(T, crc, m[q]);
-		}
-		md5_block(st, m);
-		if(b + 1 < full) {
-#pragma unroll
-			for(int q = 0; q < 16; q++) m[q] = B[q];
-			if(b + 3 < full) load_block(p4, b + 3, B);
-			if(CRC) {
-#pragma unroll
-				for(int q = 0; q < 16; q++) crc = crc_word(T, crc, m[q]);
-			}
-			md5_block(st, m);
+			for(int e = 0; e < 4; e++) m[4 * q + e] = e < 4 - C ? __ldg(p + C + k * 16 + 4 * q + e) : 0u;
 		}
 	}
 }
+// one block from the load before it and its own
+template<int C>
+__device__ __forceinline__ void md5_joined(uint32_t st[4], const uint32_t (&prev)[16], const uint32_t (&cur)[16]) {
+	uint32_t m[16];
+#pragma unroll
+	for(int q = 0; q < 16; q++) m[q] = q < C ? prev[(16 - C + q) & 15] : cur[q < C ? 0 : q - C];
+	md5_block(st, m);
+}
+template<int C>
+__device__ __forceinline__ void md5_blocks_at(uint32_t st[4], const uint32_t* p, size_t full) {
+	if(!full) return;
+	uint32_t X[16], Y[16], Z[16], W[16];
+	// X: the load before the next block's, Y: its own, Z and W: the next two
+#pragma unroll
+	for(int q = 0; q < 16; q++) X[q] = q >= 16 - C ? __ldg(p + q - (16 - C)) : 0u;
+	md5_load<C>(p, 0, full == 1, Y);
+	if(full > 1) md5_load<C>(p, 1, full == 2, Z);
+	size_t k = 0;
+	auto ahead = [&](size_t b) {
+		if(b + P2C_MD5_L2_AHEAD < full)
+			asm volatile("prefetch.global.L2 [%0];" :: "l"(p + (b + P2C_MD5_L2_AHEAD) * 16));
+	};
+	if(C == 0) {
+		for(; k + 5 <= full; k += 3) {
+			ahead(k);
+			ahead(k + 2);
+			md5_load<C>(p, k + 2, false, X);
+			md5_block(st, Y);
+			md5_load<C>(p, k + 3, false, Y);
+			md5_block(st, Z);
+			md5_load<C>(p, k + 4, false, Z);
+			md5_block(st, X);
+			// block k + 3 is in Y, k + 4 in Z
+		}
+	} else {
+		for(; k + 7 <= full; k += 4) {
+			ahead(k);
+			ahead(k + 2);
+			md5_load<C>(p, k + 2, false, W);
+			md5_joined<C>(st, X, Y);
+			md5_load<C>(p, k + 3, false, X);
+			md5_joined<C>(st, Y, Z);
+			md5_load<C>(p, k + 4, false, Y);
+			md5_joined<C>(st, Z, W);
+			md5_load<C>(p, k + 5, false, Z);
+			md5_joined<C>(st, W, X);
+			// load k + 3 is in X, k + 4 in Y, k + 5 in Z
+		}
+	}
+	for(; k < full; k++) {
+		md5_joined<C>(st, X, Y);
+#pragma unroll
+		for(int q = 0; q < 16; q++) { X[q] = Y[q]; Y[q] = Z[q]; }
+		if(k + 2 < full) md5_load<C>(p, k + 2, k + 3 == full, Z);
+	}
+}
+__device__ __forceinline__ void md5_blocks(uint32_t st[4], const uint4* p4, size_t full) {
+	md5_blocks_at<0>(st, reinterpret_cast<const uint32_t*>(p4), full);
+}
 
-// The same for a stream whose 64-byte blocks start at a 4-byte (not 16-byte)
-// boundary of memory: 32-bit loads, same two-block register pipeline and L2
-// prefetch.
+// The same from any 4-byte boundary with 32-bit loads: fewer registers, for
+// blocks of many warps.
 __device__ __forceinline__ void load_block32(const uint32_t* p, size_t b, uint32_t m[16]) {
 #pragma unroll
 	for(int q = 0; q < 16; q++) m[q] = __ldg(p + b * 16 + q);
 }
 __device__ __forceinline__ void md5_blocks32(uint32_t st[4], const uint32_t* p, size_t full) {
-	uint32_t A[16], B[16];
+	uint32_t A[16];
 	if(full > 0) load_block32(p, 0, A);
-	if(full > 1) load_block32(p, 1, B);
-	for(size_t b = 0; b < full; b += 2) {
-		uint32_t m[16];
-		if(b + P2C_MD5_L2_AHEAD < full)
+	for(size_t b = 0; b < full; b++) {
+		if((b & 1) == 0 && b + P2C_MD5_L2_AHEAD < full)
 			asm volatile("prefetch.global.L2 [%0];" :: "l"(p + (b + P2C_MD5_L2_AHEAD) * 16));
-#pragma unroll
-		for(int q = 0; q < 16; q++) m[q] = A[q];
-		if(b + 2 < full) load_block32(p, b + 2, A);
-		md5_block(st, m);
-		if(b + 1 < full) {
-#pragma unroll
-			for(int q = 0; q < 16; q++) m[q] = B[q];
-			if(b + 3 < full) load_block32(p, b + 3, B);
-			md5_block(st, m);
-		}
+		const MsgBlock m(A);
+		if(b + 1 < full) load_block32(p, b + 1, A);
+		md5_block(st, m.w);
+	}
+}
+// full 64-byte blocks from any 4-byte boundary
+__device__ __forceinline__ void md5_blocks_words(uint32_t st[4], const uint32_t* p, size_t full) {
+	switch((reinterpret_cast<uintptr_t>(p) >> 2) & 3) {
+	case 0: md5_blocks_at<0>(st, p, full); break;
+	case 1: md5_blocks_at<3>(st, p, full); break;
+	case 2: md5_blocks_at<2>(st, p, full); break;
+	default: md5_blocks_at<1>(st, p, full); break;
 	}
 }
 
@@ -218,41 +267,159 @@ __device__ __forceinline__ void md5_init(uint32_t st[4]) {
 }
 
 // ---- per-slice MD5 + CRC32 --------------------------------------------------
-// one thread per row: row i holds lens[i] bytes (or sliceBytes), hashed as if
-// zero-padded to sliceBytes.  out: 20 bytes per row.
-__global__ void __launch_bounds__(128) k_slice_hash(const uint8_t* rows, size_t pitch, unsigned n,
+// Row i holds lens[i] bytes (or sliceBytes), hashed as if zero-padded to
+// sliceBytes.  out: 20 bytes per row.
+//
+// The first blocks run the MD5s, P2C_IFSC_ROWS rows each, one row per thread:
+// the kernel's time is that chain's latency.  The CRC is linear, so the other
+// blocks compute it beside them, a row per warp: lane l takes the 16 bytes at
+// 512 k + 16 l (coalesced 512-byte loads), four registers advance 512 bytes
+// per step by table (x^4096), and the lanes' sums are joined by multiplying
+// with x^128 per lane.  2000 slices of 256 KiB + 44, every tenth one shorter:
+// 4.80 ms with the CRC in the MD5 thread, 3.26 with it in other warps of the
+// MD5 blocks (and a branch between data and padding), 2.46 so: 107 MB/s a
+// chain, which the branch for a row's partial block keeps below the 129 of
+// k_rows_md5.
+#define P2C_IFSC_ROWS 64
+#define P2C_IFSC_THREADS (32 * P2C_IFSC_ROWS / P2C_MD5_LANES)
+// tables of c x^4096 for the four bytes of a register
+struct CrcStride { uint32_t t[4][256]; };
+constexpr uint32_t crc_step_const(uint32_t c) { return (c >> 1) ^ (0xEDB88320u & (0u - (c & 1))); }
+constexpr CrcStride crc_stride() {
+	CrcStride r{};
+	for(int k = 0; k < 4; k++) {
+		uint32_t bit[8] = {};
+		for(int b = 0; b < 8; b++) {
+			uint32_t v = 1u << (8 * k + b);
+			for(int i = 0; i < 4096; i++) v = crc_step_const(v);
+			bit[b] = v;
+		}
+		for(int m = 0; m < 256; m++) {
+			uint32_t v = 0;
+			for(int b = 0; b < 8; b++) if(m >> b & 1) v ^= bit[b];
+			r.t[k][m] = v;
+		}
+	}
+	return r;
+}
+__device__ const CrcStride g_crc_stride = crc_stride();
+
+__device__ __forceinline__ uint32_t crc_stride_mul(const CrcStride& S, uint32_t r) {
+	return S.t[0][r & 255] ^ S.t[1][(r >> 8) & 255] ^ S.t[2][(r >> 16) & 255] ^ S.t[3][r >> 24];
+}
+
+// the raw CRC register of `len` bytes at the 16-byte aligned p, by one warp
+__device__ uint32_t crc_row(const CrcTabs& T, const CrcStride& S, const uint8_t* p, size_t len, int lane) {
+	const size_t steps = len / 512;
+	const uint4* p4 = reinterpret_cast<const uint4*>(p) + lane;
+	uint32_t a[4] = {0, 0, 0, 0};
+	auto add = [&](const uint4& v) {
+		a[0] = crc_stride_mul(S, a[0]) ^ v.x;
+		a[1] = crc_stride_mul(S, a[1]) ^ v.y;
+		a[2] = crc_stride_mul(S, a[2]) ^ v.z;
+		a[3] = crc_stride_mul(S, a[3]) ^ v.w;
+	};
+	size_t k = 0;
+	for(; k + 4 <= steps; k += 4) {
+		uint4 v[4];
+#pragma unroll
+		for(int u = 0; u < 4; u++) v[u] = __ldg(p4 + (k + u) * 32);
+#pragma unroll
+		for(int u = 0; u < 4; u++) add(v[u]);
+	}
+	for(; k < steps; k++) add(__ldg(p4 + k * 32));
+	// this lane's 16-byte column, then the lanes: sum over l of u_l x^(128 (31 - l))
+	uint32_t u = 0;
+#pragma unroll
+	for(int q = 0; q < 4; q++) u = crc_word(T, u, a[q]);
+	uint32_t r = 0;
+	for(int l = 0; l < 32; l++) {
+#pragma unroll
+		for(int q = 0; q < 4; q++) r = crc_word(T, r, 0);
+		r ^= __shfl_sync(0xFFFFFFFFu, u, l);
+	}
+	r ^= crc_zero_extend(0xFFFFFFFFu, steps * 512);
+	for(size_t i = steps * 512; i < len; i++) r = crc_byte(T, r, p[i]);
+	return r;
+}
+
+__global__ void __launch_bounds__(P2C_IFSC_THREADS) k_slice_hash(const uint8_t* rows, size_t pitch, unsigned n, unsigned md5Blocks,
                                                    const uint32_t* lens, size_t sliceBytes, uint8_t* out)
 {
 	__shared__ CrcTabs T;
-	crc_tabs_build(T);
-	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i >= n) return;
+	__shared__ CrcStride S;
+	const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	if(blockIdx.x >= md5Blocks) {
+		for(int i = threadIdx.x; i < 1024; i += blockDim.x) S.t[i >> 8][i & 255] = g_crc_stride.t[i >> 8][i & 255];
+		crc_tabs_build(T);
+		const unsigned i = (blockIdx.x - md5Blocks) * (P2C_IFSC_THREADS / 32) + warp;
+		if(i >= n) return;
+		const size_t len = lens ? min((size_t)lens[i], sliceBytes) : sliceBytes;
+		const uint32_t reg = crc_row(T, S, rows + (size_t)i * pitch, len, lane);
+		if(lane == 0) {
+			const uint32_t crc = ~crc_zero_extend(reg, sliceBytes - len);
+			uint8_t* o = out + (size_t)i * 20;
+			o[16] = (uint8_t)crc; o[17] = (uint8_t)(crc >> 8); o[18] = (uint8_t)(crc >> 16); o[19] = (uint8_t)(crc >> 24);
+		}
+		return;
+	}
+	const unsigned i = blockIdx.x * P2C_IFSC_ROWS + warp * P2C_MD5_LANES + lane;
+	if(lane >= P2C_MD5_LANES || i >= n) return;
 	const size_t len = lens ? min((size_t)lens[i], sliceBytes) : sliceBytes;
 	const uint8_t* p = rows + (size_t)i * pitch;
+	const uint4* p4 = reinterpret_cast<const uint4*>(p);
 	uint32_t st[4];
 	md5_init(st);
-	uint32_t crc = 0xFFFFFFFFu;
-	const size_t full = len / 64;
-	md5_blocks<true>(st, crc, T, reinterpret_cast<const uint4*>(p), full);
-	// tail bytes
+	// Every row is sliceBytes / 64 blocks and a remainder, whatever its length:
+	// blocks past its bytes are zero, taken in the same loop, so that a short
+	// row does not make its warp run the padding after the others' data.
+	const size_t own = len / 64, all = sliceBytes / 64;
+	auto block = [&](size_t k, uint32_t (&m)[16]) {
+		// loads by predicate, not under a branch that would part the warp
+#pragma unroll
+		for(int q = 0; q < 4; q++)
+			asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+			             "@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+			             : "=&r"(m[4 * q]), "=&r"(m[4 * q + 1]), "=&r"(m[4 * q + 2]), "=&r"(m[4 * q + 3])
+			             : "l"(p4 + k * 4 + q), "r"((uint32_t)(k < own)));
+		if(k == own && (len & 63)) {
+			const uint32_t rem = (uint32_t)(len - own * 64);
+#pragma unroll
+			for(int q = 0; q < 16; q++) {
+				if((uint32_t)(4 * q + 4) <= rem) m[q] = __ldg(reinterpret_cast<const uint32_t*>(p) + own * 16 + q);
+				else if((uint32_t)(4 * q) < rem)
+					for(uint32_t e = 4 * q; e < rem; e++) m[q] |= (uint32_t)p[own * 64 + e] << (8 * (e & 3));
+			}
+		}
+	};
+	uint32_t A[16], B[16];
+	block(0, A);
+	block(1, B);
+	for(size_t k = 0; k < all; k += 2) {
+		if(k + P2C_MD5_L2_AHEAD < own)
+			asm volatile("prefetch.global.L2 [%0];" :: "l"(p4 + (k + P2C_MD5_L2_AHEAD) * 4));
+		{
+			const MsgBlock m(A);
+			block(k + 2, A);
+			md5_block(st, m.w);
+		}
+		if(k + 1 < all) {
+			const MsgBlock m(B);
+			block(k + 3, B);
+			md5_block(st, m.w);
+		}
+	}
+	// the remainder of the slice (in A after an even number of blocks, else in B)
 	uint32_t tail[16];
 #pragma unroll
-	for(int q = 0; q < 16; q++) tail[q] = 0;
-	const uint32_t rem = (uint32_t)(len - full * 64);
-	for(uint32_t k = 0; k < rem; k++) {
-		uint32_t byte = p[full * 64 + k];
-		tail[k >> 2] |= byte << (8 * (k & 3));
-		crc = crc_byte(T, crc, byte);
-	}
-	md5_finish(st, tail, rem, sliceBytes - len, sliceBytes);
-	crc = ~crc_zero_extend(crc, sliceBytes - len);
+	for(int q = 0; q < 16; q++) tail[q] = (all & 1) ? B[q] : A[q];
+	md5_finish(st, tail, (uint32_t)(sliceBytes - all * 64), 0, sliceBytes);
 	uint8_t* o = out + (size_t)i * 20;
 #pragma unroll
 	for(int w = 0; w < 4; w++) {
 		o[4 * w] = (uint8_t)st[w]; o[4 * w + 1] = (uint8_t)(st[w] >> 8);
 		o[4 * w + 2] = (uint8_t)(st[w] >> 16); o[4 * w + 3] = (uint8_t)(st[w] >> 24);
 	}
-	o[16] = (uint8_t)crc; o[17] = (uint8_t)(crc >> 8); o[18] = (uint8_t)(crc >> 16); o[19] = (uint8_t)(crc >> 24);
 }
 
 int slice_hash(const void* rows, size_t pitchBytes, unsigned n, const uint32_t* dLens, size_t sliceBytes,
@@ -260,7 +427,9 @@ int slice_hash(const void* rows, size_t pitchBytes, unsigned n, const uint32_t* 
 {
 	if(!n) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
-	k_slice_hash<<<(n + 127) / 128, 128, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dLens, sliceBytes, dOut);
+	const unsigned md5Blocks = (n + P2C_IFSC_ROWS - 1) / P2C_IFSC_ROWS, per = P2C_IFSC_THREADS / 32;
+	k_slice_hash<<<md5Blocks + (n + per - 1) / per, P2C_IFSC_THREADS, 0, st>>>((const uint8_t*)rows, pitchBytes, n, md5Blocks, dLens,
+	                                                                          sliceBytes, dOut);
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
 }
@@ -335,12 +504,35 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 		const size_t take = (size_t)min((uint64_t)sliceBytes, total - done);
 		const uint8_t* p = rows + row * pitch;
 		size_t pos = 0;
-		if(tailLen == 0 && (sliceBytes % 64) == 0) {
-			// block-aligned fast path
+		if((sliceBytes % 64) == 0) {
+			// every row starts a block
 			const size_t full = take / 64;
-			uint32_t nocrc = 0;
-			md5_blocks<false>(st, nocrc, NoTabs{}, reinterpret_cast<const uint4*>(p), full);
+			md5_blocks(st, reinterpret_cast<const uint4*>(p), full);
 			pos = full * 64;
+		} else if((sliceBytes % 4) == 0 && take >= 64) {
+			// rows of whole words: the words that complete the block the last
+			// row began, then blocks from a 4-byte boundary; what is left
+			// (whole words but in a file's last row) begins the next block
+			const uint32_t* d32 = reinterpret_cast<const uint32_t*>(p);
+			if(tailLen) {
+				const uint32_t have = tailLen >> 2;
+#pragma unroll
+				for(uint32_t q = 0; q < 16; q++) if(q >= have) tail[q] = __ldg(d32 + q - have);
+				md5_block(st, tail);
+				pos = 64 - tailLen;
+				tailLen = 0;
+#pragma unroll
+				for(int q = 0; q < 16; q++) tail[q] = 0;
+			}
+			const size_t full = (take - pos) / 64;
+			if(MAXT > 32) md5_blocks32(st, d32 + pos / 4, full);
+			else md5_blocks_words(st, d32 + pos / 4, full);
+			pos += full * 64;
+			const uint32_t words = (uint32_t)(take - pos) / 4;
+#pragma unroll
+			for(uint32_t q = 0; q < 16; q++) if(q < words) tail[q] = __ldg(d32 + pos / 4 + q);
+			tailLen = 4 * words;
+			pos += tailLen;
 		}
 		for(; pos < take; pos++) {
 			tail[tailLen >> 2] |= (uint32_t)p[pos] << (8 * (tailLen & 3));
@@ -423,22 +615,23 @@ __device__ __forceinline__ bool hs_wait(uint32_t bar, uint32_t parity) {
 }
 
 template<int NT>
-__global__ void __launch_bounds__(NT) k_file_md5_staged(const uint8_t* __restrict__ rows, size_t pitch, unsigned nFiles,
+__global__ void __launch_bounds__(NT * 32 / P2C_MD5_LANES) k_file_md5_staged(const uint8_t* __restrict__ rows, size_t pitch, unsigned nFiles,
                                                         const uint64_t* __restrict__ fileLen,
                                                         const uint32_t* __restrict__ firstRow, size_t sliceBytes,
                                                         uint8_t* __restrict__ out, const uint32_t* __restrict__ outIndex)
 {
 	extern __shared__ __align__(128) uint8_t smem[];
-	const unsigned t = threadIdx.x;
+	const unsigned t = (threadIdx.x >> 5) * P2C_MD5_LANES + (threadIdx.x & 31);
+	const bool mine = (threadIdx.x & 31) < P2C_MD5_LANES;
 	const unsigned f = blockIdx.x * NT + t;
 	uint8_t* ring = smem + (size_t)t * P2C_STG_STRIDE;
 	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)NT * P2C_STG_STRIDE) + t * P2C_STG_NS;
 	const uint32_t ringA = hs_saddr(ring), barA = hs_saddr(bars);
-	for(int k = 0; k < P2C_STG_NS; k++)
+	if(mine) for(int k = 0; k < P2C_STG_NS; k++)
 		asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barA + 8 * k) : "memory");
 	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	__syncthreads();
-	if(f >= nFiles) return;
+	if(!mine || f >= nFiles) return;
 
 	const uint64_t total = fileLen[f];
 	const uint8_t* base = rows + (size_t)firstRow[f] * pitch;
@@ -545,11 +738,11 @@ int file_md5_staged(const void* rows, size_t pitchBytes, unsigned nFiles, const 
 	const size_t smem = (size_t)filesPerBlock * (P2C_STG_STRIDE + 8 * P2C_STG_NS);
 	if(filesPerBlock == 32) {
 		P2C_CUDA_TRY(cudaFuncSetAttribute(k_file_md5_staged<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		k_file_md5_staged<32><<<(nFiles + 31) / 32, 32, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
+		k_file_md5_staged<32><<<(nFiles + 31) / 32, 32 * 32 / P2C_MD5_LANES, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
 		                                                             dFirstRow, sliceBytes, dOut, dOutIndex);
 	} else {
 		P2C_CUDA_TRY(cudaFuncSetAttribute(k_file_md5_staged<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		k_file_md5_staged<64><<<(nFiles + 63) / 64, 64, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
+		k_file_md5_staged<64><<<(nFiles + 63) / 64, 64 * 32 / P2C_MD5_LANES, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
 		                                                             dFirstRow, sliceBytes, dOut, dOutIndex);
 	}
 	P2C_CUDA_TRY(cudaGetLastError());
@@ -566,11 +759,11 @@ int hash_error_take() {
 // ---- MD5 of equal-length rows (recovery packets; MD5Multi, hasher/hasher.h:33-56)
 // row i: prefix[i] (prefixLen bytes, host-assembled packet header) followed by
 // dataLen bytes of row data.  One thread per row.
-__global__ void __launch_bounds__(128) k_rows_md5(const uint8_t* rows, size_t pitch, unsigned n, size_t dataLen,
+__global__ void __launch_bounds__(32 * 32 / P2C_MD5_LANES) k_rows_md5(const uint8_t* rows, size_t pitch, unsigned n, size_t dataLen,
                                                  const uint8_t* prefix, unsigned prefixLen, uint8_t* out)
 {
-	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-	if(i >= n) return;
+	const unsigned lane = threadIdx.x & 31, i = blockIdx.x * 32 + (threadIdx.x >> 5) * P2C_MD5_LANES + lane;
+	if(lane >= P2C_MD5_LANES || i >= n) return;
 	uint32_t st[4];
 	md5_init(st);
 	uint32_t tail[16];
@@ -585,8 +778,7 @@ __global__ void __launch_bounds__(128) k_rows_md5(const uint8_t* rows, size_t pi
 	const uint8_t* p = rows + (size_t)i * pitch;
 	size_t pos = 0;
 	if(tailLen == 0) {
-		uint32_t nocrc = 0;
-		md5_blocks<false>(st, nocrc, NoTabs{}, reinterpret_cast<const uint4*>(p), dataLen / 64);
+		md5_blocks(st, reinterpret_cast<const uint4*>(p), dataLen / 64);
 		pos = dataLen / 64 * 64;
 	} else if(tailLen % 4 == 0 && dataLen >= 64 - tailLen) {
 		// a prefix of whole words (the 36-byte packet header): complete its
@@ -600,7 +792,7 @@ __global__ void __launch_bounds__(128) k_rows_md5(const uint8_t* rows, size_t pi
 		tailLen = 0;
 		pos = (size_t)need * 4;
 		const size_t full = (dataLen - pos) / 64;
-		md5_blocks32(st, d32 + need, full);
+		md5_blocks_words(st, d32 + need, full);
 		pos += full * 64;
 	}
 	for(; pos < dataLen; pos++) {
@@ -621,7 +813,9 @@ int rows_md5(const void* rows, size_t pitchBytes, unsigned n, size_t dataLen, co
 {
 	if(!n) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
-	k_rows_md5<<<(n + 127) / 128, 128, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dataLen, dPrefix, prefixLen, dOut);
+	// 32 rows per block: a chain's latency is what counts, so the rows are
+	// spread over the SMs
+	k_rows_md5<<<(n + 31) / 32, 32 * 32 / P2C_MD5_LANES, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dataLen, dPrefix, prefixLen, dOut);
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
 }

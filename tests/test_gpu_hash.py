@@ -140,3 +140,64 @@ def test_packed_file_md5_matches_unpacked():
     a = int(job.first_row[f])
     data = rows[a:a + (lens[f] + S - 1) // S, :S].reshape(-1)[:lens[f]]
     assert outs[0][16 * f:16 * f + 16].tobytes() == O.md5(data)
+
+
+@pytest.mark.parametrize("S", [4, 60, 68, 72, 76, 1020, 4100, 8200, 12300, 20484])
+def test_file_md5_of_rows_that_split_blocks(S):
+    """Slice sizes of whole words that are no multiple of a 64-byte block: rows
+    begin inside a block, at every 16-byte phase, with whole and partial last
+    rows; one file per block, packed and pooled."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    lengths = [1, 63, 64, S - 1, S, S + 1, 2 * S + 3, 3 * S, 5 * S + S // 2, 9 * S - 2]
+    files = [synth.slice_bytes(900 + S, k, n) for k, n in enumerate(lengths)]
+    d, pitch, lens, first, nrows = _rows_from_files(torch, files, S)
+    want = b"".join(hashlib.md5(f.tobytes()).digest() for f in files)
+    flen = torch.tensor(lengths, dtype=torch.int64, device="cuda")
+    d_first = torch.from_numpy(first.view(np.int32)).cuda()
+    for call in (L.par2cuda_file_md5, L.par2cuda_file_md5_packed,
+                 lambda *a: L.par2cuda_file_md5_pooled(*a[:7], 64, a[7])):
+        md5 = torch.zeros(16 * len(files), dtype=torch.uint8, device="cuda")
+        _lib.check(call(d.data_ptr(), pitch, len(files), flen.data_ptr(), d_first.data_ptr(), S, md5.data_ptr(), None), "file_md5")
+        torch.cuda.synchronize()
+        assert md5.cpu().numpy().tobytes() == want
+
+
+@pytest.mark.parametrize("prefix", [0, 4, 8, 12, 16, 36, 60, 64, 100])
+@pytest.mark.parametrize("data", [0, 27, 28, 60, 92, 128, 1000, 4097])
+def test_rows_md5_prefixes(prefix, data):
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    n = 35
+    pitch = L.par2cuda_row_pitch_bytes(max(data, 2))
+    rows = synth.slices(77, 0, n, pitch)
+    pre = synth.slices(78, 0, n, max(prefix, 1))[:, :prefix]
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_pre = torch.from_numpy(np.ascontiguousarray(pre)).cuda() if prefix else None
+    out = torch.zeros(16 * n, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_rows_md5(d.data_ptr(), pitch, n, data, d_pre.data_ptr() if prefix else None, prefix, out.data_ptr(),
+                                   None), "rows_md5")
+    torch.cuda.synchronize()
+    want = b"".join(hashlib.md5(pre[i].tobytes() + rows[i, :data].tobytes()).digest() for i in range(n))
+    assert out.cpu().numpy().tobytes() == want
+
+
+@pytest.mark.parametrize("n", [1, 64, 65, 150])
+def test_ifsc_lengths_around_the_crc_step(n):
+    """Row lengths around the 512-byte step of the CRC and its four-step loop."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    S = 5000
+    pitch = L.par2cuda_row_pitch_bytes(S)
+    edges = [0, 1, 511, 512, 513, 1535, 2047, 2048, 2049, 2560, 4095, 4096, 4608, 4999, 5000]
+    lens = np.array([edges[k % len(edges)] for k in range(n)], dtype=np.uint32)
+    rows = synth.slices(79, 0, n, pitch)
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_lens = torch.from_numpy(lens.view(np.int32)).cuda()
+    out = torch.zeros(n * 20, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_slice_hash(d.data_ptr(), pitch, n, d_lens.data_ptr(), S, out.data_ptr(), None), "slice_hash")
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(n, 20)
+    for i in range(n):
+        padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
+        assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
