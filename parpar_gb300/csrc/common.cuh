@@ -47,19 +47,6 @@ __device__ __forceinline__ uint16_t gf_mul_tab(const GfTables& t, uint16_t a, ui
 	return t.exp[(uint32_t)t.log[a] + t.log[b]];
 }
 
-// per-lane multiply of a 4-lane checksum block by 2^e
-__device__ __forceinline__ uint64_t cksum_mul_exp(const GfTables& t, uint64_t ck, uint32_t e) {
-	uint64_t r = 0;
-	uint32_t em = e % 65535u;
-#pragma unroll
-	for(int l = 0; l < 4; l++) {
-		uint16_t v = (uint16_t)(ck >> (16 * l));
-		uint16_t p = v ? t.exp[(uint32_t)t.log[v] + em] : 0;
-		r |= (uint64_t)p << (16 * l);
-	}
-	return r;
-}
-
 } // namespace p2c
 
 // error plumbing shared by the host-side files

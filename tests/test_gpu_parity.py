@@ -246,6 +246,33 @@ def test_device_checksum_detects_corruption():
     assert flags.tolist() == [1, 1, 1, 1, 0, 1]
 
 
+@pytest.mark.parametrize("n,S", [
+    (3, 2), (2, 126), (5, 130),      # within and just past one lane's 128 bytes
+    (3, 4094), (3, 4098),            # a warp's 4096
+    (2, 16384), (2, 16392),          # a CTA's 16 384, and one block more
+    (1, 3_000_010),                  # many CTAs to a row
+    (70, 1_400_012),                 # more than 128 bytes per lane
+])
+def test_device_checksum_at_its_edges(n, S):
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    rows, pw = _dev_rows(torch, n, S, S)
+    lens = [(S, S - 1, S // 2 | 1, 0, min(S, 15))[i % 5] for i in range(n)]
+    d_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    ck = torch.zeros(n * 8, dtype=torch.uint8, device="cuda")
+    flags = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_rows_checksum(rows.data_ptr(), pw, n, d_lens.data_ptr(), S, 0, None, ck.data_ptr(), None), "ck")
+    _lib.check(L.par2cuda_rows_checksum(rows.data_ptr(), pw, n, None, S, 1, flags.data_ptr(), ck.data_ptr(), None), "verify")
+    torch.cuda.synchronize()
+    host = synth.slices(S, 0, n, S)
+    got = rows.cpu().numpy().view(np.uint8)
+    Sp = (S + 7) // 8 * 8
+    for i, l in enumerate(lens):
+        assert np.array_equal(got[i, :l], host[i, :l]) and not got[i, l:Sp].any() and not got[i, Sp + 8:].any()
+        assert int.from_bytes(got[i, Sp:Sp + 8].tobytes(), "little") == O.cksum(host[i, :l], S)
+    assert flags.tolist() == [1] * n
+
+
 # ------------------------------------------------------------ full-size properties
 def _sampled_check(torch, d_in, pw, n, d_rec, R, S, exps, samples=48, seed=0):
     """rec[r][w] == sum_i c(i, e_r) * in[i][w] at sampled (r, w)."""
