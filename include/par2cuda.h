@@ -42,6 +42,7 @@ typedef struct par2cuda_ctx par2cuda_ctx;
 /* status / verdict callback: status >= 0 on success (get_output: 1 = checksum
  * valid, 0 = invalid), negative on error */
 typedef void (*par2cuda_done_fn)(void* user, int status);
+typedef void (*par2cuda_done_group_fn)(void* const* users, const int* statuses, unsigned n);
 /* batch-completion progress callback (IPAR2ProcBackend::progressCb,
  * gf16/controller.h:93, called from _notifyProc gf16/controller_cpu.cpp:627-645) */
 typedef void (*par2cuda_progress_fn)(void* user, unsigned numInputs);
@@ -97,6 +98,14 @@ int par2cuda_set_current_slice_size(par2cuda_ctx* ctx, size_t size);
 /* setRecoverySlices(numSlices, exponents) gf16/controller.h:167; exponents
  * may be NULL when every input is added with explicit coefficients */
 int par2cuda_set_recovery_slices(par2cuda_ctx* ctx, unsigned num_slices, const uint16_t* exponents);
+/* Completions in groups: with fn set (before the first input), the callbacks
+ * given to addInput and getOutput are not called one by one; fn(users, statuses,
+ * n) gets what each would have been called with, in the same order, and `cb`
+ * says only whether the completion is wanted.  For hosts to whom a call is
+ * expensive (an interpreter lock to take): nothing is held back, a group is
+ * what completed while the one before was handled.  NULL (the default): one by
+ * one. */
+int par2cuda_set_done_group(par2cuda_ctx* ctx, par2cuda_done_group_fn fn);
 /* setMinInputBatchSize(size) gf16/controller.h:212-214 */
 int par2cuda_set_min_input_batch(par2cuda_ctx* ctx, unsigned size);
 /* setProgressCb gf16/controller.h:162-164 */

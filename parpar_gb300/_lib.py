@@ -12,6 +12,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libpar2cuda.so")
 
 DONE_FN = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_int)
+DONE_GROUP_FN = ctypes.CFUNCTYPE(None, ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_int), ctypes.c_uint)
 PROGRESS_FN = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_uint)
 
 ADD_OK, ADD_OK_BUSY, ADD_FULL = 0, 1, 2
@@ -60,6 +61,7 @@ SIGNATURES = [
     ("par2cuda_set_current_slice_size", _i, [_vp, _sz]),
     ("par2cuda_set_recovery_slices", _i, [_vp, _u, _vp]),
     ("par2cuda_set_min_input_batch", _i, [_vp, _u]),
+    ("par2cuda_set_done_group", _i, [_vp, DONE_GROUP_FN]),
     ("par2cuda_set_progress_cb", _i, [_vp, PROGRESS_FN, _vp]),
     ("par2cuda_can_add", _i, [_vp]),
     ("par2cuda_wait_for_add", _i, [_vp]),

@@ -57,6 +57,7 @@ int par2cuda_set_recovery_slices(par2cuda_ctx* ctx, unsigned n, const uint16_t* 
 	return ctx->eng->set_recovery_slices(n, exps);
 }
 int par2cuda_set_min_input_batch(par2cuda_ctx* ctx, unsigned size) { P2C_CTX_CHECK(ctx); ctx->eng->set_min_input_batch(size); return 0; }
+int par2cuda_set_done_group(par2cuda_ctx* ctx, par2cuda_done_group_fn fn) { P2C_CTX_CHECK(ctx); ctx->eng->set_done_group(fn); return 0; }
 int par2cuda_set_progress_cb(par2cuda_ctx* ctx, par2cuda_progress_fn fn, void* user) { P2C_CTX_CHECK(ctx); ctx->eng->set_progress(fn, user); return 0; }
 int par2cuda_can_add(par2cuda_ctx* ctx) { P2C_CTX_CHECK(ctx); return ctx->eng->can_add(); }
 int par2cuda_wait_for_add(par2cuda_ctx* ctx) { P2C_CTX_CHECK(ctx); return ctx->eng->wait_for_add(); }

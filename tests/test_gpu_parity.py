@@ -246,6 +246,38 @@ def test_device_checksum_detects_corruption():
     assert flags.tolist() == [1, 1, 1, 1, 0, 1]
 
 
+@pytest.mark.parametrize("n,S,batch,pinned", [(1, 2, 0, False), (40, 1000, 8, False), (40, 1000, 8, True), (300, 100000, 64, True)])
+@pytest.mark.filterwarnings("ignore::pytest.PytestUnraisableExceptionWarning")
+def test_completions_come_once_and_in_order(n, S, batch, pinned):
+    # however they are grouped, and although one of them raises
+    torch = pytest.importorskip("torch")
+    R = 5
+    host_in = torch.zeros((n, S), dtype=torch.uint8, pin_memory=pinned)
+    host_in.copy_(torch.from_numpy(synth.slices(3, 0, n, S)))
+    host_out = torch.zeros((R, S), dtype=torch.uint8, pin_memory=pinned)
+    g = GfProc(S, input_batchsize=batch)
+    g.set_recovery_slices(range(R))
+    for _ in range(2):
+        seen, verdicts = [], []
+
+        def done(i, buf):
+            seen.append(i)
+            if i == 1:
+                raise RuntimeError("a failing completion")
+        for i in range(n):
+            while not g.add(i, host_in[i], done):
+                _lib.load().par2cuda_wait_for_add(g._ctx)
+        g.end_sync()
+        assert seen == list(range(n))
+        for r in range(R):
+            g.get(r, host_out[r], lambda i, ok, out: verdicts.append((i, ok)))
+        g.sync()
+        assert verdicts == [(r, True) for r in range(R)]
+        want = O.recover(host_in.numpy(), np.full(n, S), range(n), range(R))
+        assert np.array_equal(host_out.numpy(), want)
+    g.close()
+
+
 @pytest.mark.parametrize("n,S", [
     (3, 2), (2, 126), (5, 130),      # within and just past one lane's 128 bytes
     (3, 4094), (3, 4098),            # a warp's 4096
