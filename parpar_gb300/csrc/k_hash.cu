@@ -277,10 +277,12 @@ __device__ __forceinline__ void md5_init(uint32_t st[4]) {
 // per step by table (x^4096), and the lanes' sums are joined by multiplying
 // with x^128 per lane.  2000 slices of 256 KiB + 44, every tenth one shorter:
 // 4.80 ms with the CRC in the MD5 thread, 3.26 with it in other warps of the
-// MD5 blocks (and a branch between data and padding), 2.46 so: 107 MB/s a
-// chain, which the branch for a row's partial block keeps below the 129 of
-// k_rows_md5.
-#define P2C_IFSC_ROWS 64
+// MD5 blocks (and a branch between data and padding), 2.46 beside them, and
+// 1.98 (132 MB/s a chain, of the 170 that the chain's own latency allows) with
+// rows' partial blocks out of the loop (2.26) and 16 rows a block, so that two
+// MD5 warps seldom share a scheduler (32 rows: 2.13).  10 000 slices of 64 KiB
+// 1.01 -> 0.81 ms.
+#define P2C_IFSC_ROWS 16
 #define P2C_IFSC_THREADS (32 * P2C_IFSC_ROWS / P2C_MD5_LANES)
 // tables of c x^4096 for the four bytes of a register
 struct CrcStride { uint32_t t[4][256]; };
@@ -343,6 +345,8 @@ __device__ uint32_t crc_row(const CrcTabs& T, const CrcStride& S, const uint8_t*
 	return r;
 }
 
+__device__ const uint4 g_md5_zero[4] = {};
+
 __global__ void __launch_bounds__(P2C_IFSC_THREADS) k_slice_hash(const uint8_t* rows, size_t pitch, unsigned n, unsigned md5Blocks,
                                                    const uint32_t* lens, size_t sliceBytes, uint8_t* out)
 {
@@ -364,6 +368,7 @@ __global__ void __launch_bounds__(P2C_IFSC_THREADS) k_slice_hash(const uint8_t* 
 		return;
 	}
 	const unsigned i = blockIdx.x * P2C_IFSC_ROWS + warp * P2C_MD5_LANES + lane;
+	const uint32_t act = __ballot_sync(0xFFFFFFFFu, lane < P2C_MD5_LANES && i < n);
 	if(lane >= P2C_MD5_LANES || i >= n) return;
 	const size_t len = lens ? min((size_t)lens[i], sliceBytes) : sliceBytes;
 	const uint8_t* p = rows + (size_t)i * pitch;
@@ -371,49 +376,75 @@ __global__ void __launch_bounds__(P2C_IFSC_THREADS) k_slice_hash(const uint8_t* 
 	uint32_t st[4];
 	md5_init(st);
 	// Every row is sliceBytes / 64 blocks and a remainder, whatever its length:
-	// blocks past its bytes are zero, taken in the same loop, so that a short
-	// row does not make its warp run the padding after the others' data.
-	const size_t own = len / 64, all = sliceBytes / 64;
-	auto block = [&](size_t k, uint32_t (&m)[16]) {
-		// loads by predicate, not under a branch that would part the warp
+	// blocks past its bytes are zero, taken in the same loop (from an address
+	// of zeros), so that a short row does not make its warp run the padding
+	// after the others' data.  A block that a row fills in part is put together
+	// when it is used: the loop runs up to the pair of blocks that holds the
+	// next one of any of the warp's rows, without a test per block.
+	const uint32_t own = (uint32_t)(len / 64), all = (uint32_t)(sliceBytes / 64);
+	const uint4* const zero = g_md5_zero;
+	auto block = [&](uint32_t k, uint32_t (&m)[16]) {
+		const uint4* src = k < own ? p4 + (size_t)k * 4 : zero;
 #pragma unroll
-		for(int q = 0; q < 4; q++)
-			asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
-			             "@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-			             : "=&r"(m[4 * q]), "=&r"(m[4 * q + 1]), "=&r"(m[4 * q + 2]), "=&r"(m[4 * q + 3])
-			             : "l"(p4 + k * 4 + q), "r"((uint32_t)(k < own)));
-		if(k == own && (len & 63)) {
-			const uint32_t rem = (uint32_t)(len - own * 64);
+		for(int q = 0; q < 4; q++) {
+			const uint4 v = __ldg(src + q);
+			m[4 * q] = v.x; m[4 * q + 1] = v.y; m[4 * q + 2] = v.z; m[4 * q + 3] = v.w;
+		}
+	};
+	auto cut = [&](uint32_t k, uint32_t (&m)[16]) {
+		if(k == own) {
+			const uint32_t rem = (uint32_t)(len - (size_t)own * 64);
 #pragma unroll
 			for(int q = 0; q < 16; q++) {
-				if((uint32_t)(4 * q + 4) <= rem) m[q] = __ldg(reinterpret_cast<const uint32_t*>(p) + own * 16 + q);
+				if((uint32_t)(4 * q + 4) <= rem) m[q] = __ldg(reinterpret_cast<const uint32_t*>(p4 + (size_t)own * 4) + q);
 				else if((uint32_t)(4 * q) < rem)
-					for(uint32_t e = 4 * q; e < rem; e++) m[q] |= (uint32_t)p[own * 64 + e] << (8 * (e & 3));
+					for(uint32_t e = 4 * q; e < rem; e++) m[q] |= (uint32_t)p[(size_t)own * 64 + e] << (8 * (e & 3));
 			}
 		}
 	};
 	uint32_t A[16], B[16];
 	block(0, A);
 	block(1, B);
-	for(size_t k = 0; k < all; k += 2) {
-		if(k + P2C_MD5_L2_AHEAD < own)
-			asm volatile("prefetch.global.L2 [%0];" :: "l"(p4 + (k + P2C_MD5_L2_AHEAD) * 4));
+	uint32_t k = 0;
+	for(;;) {
+		// the next block of which some lane has a part (or the last)
+		const uint32_t mine = own >= k && own < all ? own : all;
+		const uint32_t stop = __reduce_min_sync(act, mine) & ~1u;
+		for(; k < stop; k += 2) {
+			if(k + P2C_MD5_L2_AHEAD < own)
+				asm volatile("prefetch.global.L2 [%0];" :: "l"(p4 + (size_t)(k + P2C_MD5_L2_AHEAD) * 4));
+			{
+				const MsgBlock m(A);
+				block(k + 2, A);
+				md5_block(st, m.w);
+			}
+			{
+				const MsgBlock m(B);
+				block(k + 3, B);
+				md5_block(st, m.w);
+			}
+		}
+		if(k >= all) break;
 		{
+			cut(k, A);
 			const MsgBlock m(A);
 			block(k + 2, A);
 			md5_block(st, m.w);
 		}
 		if(k + 1 < all) {
+			cut(k + 1, B);
 			const MsgBlock m(B);
 			block(k + 3, B);
 			md5_block(st, m.w);
 		}
+		k += 2;
 	}
 	// the remainder of the slice (in A after an even number of blocks, else in B)
 	uint32_t tail[16];
 #pragma unroll
 	for(int q = 0; q < 16; q++) tail[q] = (all & 1) ? B[q] : A[q];
-	md5_finish(st, tail, (uint32_t)(sliceBytes - all * 64), 0, sliceBytes);
+	cut(all, tail);
+	md5_finish(st, tail, (uint32_t)(sliceBytes - (size_t)all * 64), 0, sliceBytes);
 	uint8_t* o = out + (size_t)i * 20;
 #pragma unroll
 	for(int w = 0; w < 4; w++) {

@@ -201,3 +201,25 @@ def test_ifsc_lengths_around_the_crc_step(n):
     for i in range(n):
         padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
         assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
+
+
+@pytest.mark.parametrize("S", [4, 60, 64, 68, 128, 192, 196, 256, 1020, 1088])
+def test_ifsc_partial_blocks_of_neighbouring_rows(S):
+    """Rows of one warp that end in different blocks: an even and an odd number of blocks, with and without a remainder,
+    each row's last block empty, begun, whole, or shared by a pair."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    n = 35                            # two blocks of 16 rows and a part of one
+    pitch = L.par2cuda_row_pitch_bytes(S)
+    lens = np.array([(S, 0, S - 1, 64 * (i % 5), 64 * (i % 7) + i, S // 2, 3 * i)[i % 7] for i in range(n)])
+    lens = np.minimum(lens, S).astype(np.uint32)
+    rows = synth.slices(80, 0, n, pitch)
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_lens = torch.from_numpy(lens.view(np.int32)).cuda()
+    out = torch.zeros(n * 20, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_slice_hash(d.data_ptr(), pitch, n, d_lens.data_ptr(), S, out.data_ptr(), None), "slice_hash")
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(n, 20)
+    for i in range(n):
+        padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
+        assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
