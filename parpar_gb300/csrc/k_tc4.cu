@@ -1029,11 +1029,42 @@ struct T4Plan {
 	unsigned BN, nTiles;   // columns per tile, column tiles
 	size_t bBytes;         // prepared coefficients
 	size_t pairBytes;      // compact A of 256 words
-	size_t chunkWords;     // words per chunk
+	unsigned chunks;       // chunks of words, one preparation and one GEMM launch each
+	unsigned nBig;         // the first nBig hold bigWords, the others restWords, the last what is left
+	size_t bigWords, restWords;
+	bool fits;             // in the scratch
 	double cost;           // modelled clocks of a CTA pair for the whole call
 };
 
-static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t chunkWords, unsigned nPairsSM) {
+// Sizes of the chunks.  A launch takes whole waves of the grid, however few
+// tiles the last one has, and as many chunks of one size often end just past a
+// wave: 2000 x 200 x 2 MiB, 16 chunks of 3.4 waves cost 64.  Where two sizes,
+// one of whole waves and one above it, come to fewer waves for as many chunks,
+// they are taken (58 there: 11.39 -> 10.66 ms; 4096 x 4096 x 256 KiB, 125 -> 122
+// waves, 28.08 -> 27.63; 4096 x 240 x 256 KiB 3.05 -> 2.77).
+static unsigned t4_chunks(T4Plan& pl, size_t nWords, size_t cw, size_t capPairs, unsigned nPairsSM) {
+	const size_t pairWords = 2 * T4_ROWS;
+	auto waves = [&](size_t pairs) { return (pairs * pl.nTiles + nPairsSM - 1) / nPairsSM; };
+	pl.chunks = pl.nBig = (unsigned)((nWords + cw - 1) / cw);
+	pl.bigWords = pl.restWords = cw;
+	const size_t lastWords = nWords - (size_t)(pl.chunks - 1) * cw;
+	const size_t even = (pl.chunks - 1) * waves((cw + pairWords - 1) / pairWords) + waves((lastWords + pairWords - 1) / pairWords);
+	const size_t total = (nWords + pairWords - 1) / pairWords, n = pl.chunks;
+	const size_t lo = total / n * pl.nTiles / nPairsSM;      // whole waves of an average chunk
+	if(n < 2 || !lo) return (unsigned)even;
+	const size_t a = lo * nPairsSM / pl.nTiles, b = std::min((lo + 1) * nPairsSM / pl.nTiles, capPairs);
+	if(!a || b <= a) return (unsigned)even;
+	const size_t big = a * n >= total ? 0 : (total - a * n + b - a - 1) / (b - a);
+	if(big > n) return (unsigned)even;
+	const size_t mixed = big * waves(b) + (n - big) * waves(a), spare = big * b + (n - big) * a - total;
+	if(mixed >= even || spare >= (big < n ? a : b)) return (unsigned)even;
+	pl.nBig = (unsigned)big;
+	pl.bigWords = b * pairWords;
+	pl.restWords = a * pairWords;
+	return (unsigned)mixed;
+}
+
+static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t cw, size_t scratchBytes, unsigned nPairsSM) {
 	T4Plan pl;
 	const unsigned cpr = form == 4 ? 4 : 1;
 	const unsigned cap = tc4_shape_for(0) == 2 ? 128 : T4_MAXN;
@@ -1046,21 +1077,23 @@ static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t 
 	pl.nTiles = (unsigned)((cols + pl.BN - 1) / pl.BN);
 	pl.bBytes = round_up((size_t)pl.nTiles * pl.P * pl.U * pl.BN * 48, 1024);
 	pl.pairBytes = (size_t)2 * pl.P * pl.U * T4_UNIT_Q;
-	pl.chunkWords = chunkWords;
+	const size_t fixed = T4_HDR_BYTES + pl.bBytes, needed = (cw + 2 * T4_ROWS - 1) / (2 * T4_ROWS) * pl.pairBytes;
+	pl.fits = scratchBytes >= fixed + needed;
+	if(!pl.fits) return pl;
+	const double waves = t4_chunks(pl, nWords, cw, (scratchBytes - fixed) / pl.pairBytes, nPairsSM);
 	// Fitted to GB300 times: a pass costs ~1000 clocks (its signals between
 	// the roles), ~100 per stage and the MMAs (0.5 per column, at least 68);
-	// a chunk takes whole waves of the grid; preparing an input word moves
+	// a launch takes whole waves of the grid; preparing an input word moves
 	// 2 + 3.5 (form 4) or 2 + 7.9 bytes at 6.7 clocks of the grid per byte
 	// and pair tile.  Form 1 wins where the passes are long and the columns
-	// fill its tiles: 4096 x 4096 x 256 KiB 27.6 against 42.5 ms, 2000 x 200 x
-	// 2 MiB 10.8 against 12.2; form 4 for 1000 x 100 x 1 MiB 2.0 against 3.2,
-	// 300 x 45 x 4 MiB 2.1 against 6.1.
+	// fill its tiles (ms, form 1 against form 4): 4096 x 4096 x 256 KiB 27.6
+	// and 43.6, 2000 x 200 x 2 MiB 10.7 and 12.1, 1000 x 480 x 1 MiB 5.7 and
+	// 6.0; form 4 for 1000 x 300 x 1 MiB 5.4 and 3.9, 2000 x 100 x 2 MiB 10.1
+	// and 7.2, 500 x 480 x 1 MiB 4.4 and 3.6.
 	const double stages = (pl.U + T4_SU - 1) / T4_SU;
 	const double pass = 1000 + 100 * stages + pl.U * std::max(0.5 * pl.BN, 68.0);
-	const size_t chunks = (nWords + chunkWords - 1) / chunkWords;
-	const size_t pairs = (std::min(chunkWords, nWords) + 2 * T4_ROWS - 1) / (2 * T4_ROWS);
-	const double waves = (double)((pairs * pl.nTiles + nPairsSM - 1) / nPairsSM);
-	pl.cost = chunks * (waves * pl.P * pass + 6.7 * nIn * (2 + (form == 4 ? 3.5 : 7.9)) * pairs / nPairsSM);
+	const double pairs = (double)((nWords + 2 * T4_ROWS - 1) / (2 * T4_ROWS));
+	pl.cost = waves * pl.P * pass + 6.7 * nIn * (2 + (form == 4 ? 3.5 : 7.9)) * pairs / nPairsSM;
 	return pl;
 }
 
@@ -1087,7 +1120,7 @@ static size_t t4_min_scratch(unsigned R, unsigned nIn) {
 
 // false: too little scratch.  The number of word chunks is that of expanded
 // planes of 8 bytes per word and (padded) input in the given scratch, the
-// launch count callers are told; chunks are of even size within that number.
+// launch count callers are told; t4_chunks lays them out within that number.
 static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM) {
 	if(scratchBytes < t4_min_scratch(R, nIn)) return false;
 	size_t cw = (scratchBytes - T4_HDR_BYTES - t4_bbytes(R, nIn)) / t4_kbytes(nIn) / T4_ROWS * T4_ROWS;
@@ -1097,10 +1130,9 @@ static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t 
 	if(even <= cw && (nWords + even - 1) / even == chunks) cw = even;
 	bool have = false;
 	for(int form : {4, 1}) {
-		const T4Plan c = t4_form(form, R, nIn, nWords, cw, nPairsSM);
-		const size_t pairs = (cw + 2 * T4_ROWS - 1) / (2 * T4_ROWS);
+		const T4Plan c = t4_form(form, R, nIn, nWords, cw, scratchBytes, nPairsSM);
 		if(form == 1 && c.U < T4_SU) continue;       // its passes are single stages or more
-		if(scratchBytes < T4_HDR_BYTES + c.bBytes + pairs * c.pairBytes) continue;
+		if(!c.fits) continue;
 		if(!have || c.cost < pl.cost) pl = c;
 		have = true;
 	}
@@ -1118,7 +1150,7 @@ static int t4_pairs_on_device(unsigned* out) {
 unsigned tc4_launches(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes) {
 	T4Plan pl;
 	if(!R || !nWords || !nIn || !t4_plan(pl, R, nIn, nWords, scratchBytes, 76)) return 0;
-	return 1 + 2 * (unsigned)((nWords + pl.chunkWords - 1) / pl.chunkWords);   // coefficients, then per chunk: inputs + GEMM
+	return 1 + 2 * pl.chunks;   // coefficients, then per chunk: inputs + GEMM
 }
 
 typedef decltype(&k_tc4_gemm<4, 0>) T4Gemm;
@@ -1163,8 +1195,9 @@ static int t4_run(const T4Plan& pl, const uint16_t* in, size_t inPitch, unsigned
 	const unsigned rings = t4_rings(isShort ? T4_SU / pl.U * pl.U : T4_SU, pl.BN);
 	if(!rings) { set_error("tensor method (mxf4): no stage layout for %u columns", pl.BN); return -1; }
 	unsigned base = 0;
-	for(size_t w0 = 0; w0 < nWords; w0 += pl.chunkWords) {
-		const size_t wEnd = std::min(nWords, w0 + pl.chunkWords);
+	size_t w0 = 0, wEnd;
+	for(unsigned chunk = 0; chunk < pl.chunks; chunk++, w0 = wEnd) {
+		wEnd = std::min(nWords, w0 + (chunk < pl.nBig ? pl.bigWords : pl.restWords));
 		const unsigned mTiles = (unsigned)((wEnd - w0 + 2 * T4_ROWS - 1) / (2 * T4_ROWS));
 		const unsigned groups = (nIn + 31) / 32;
 		const size_t items = (size_t)mTiles * 2 * groups;

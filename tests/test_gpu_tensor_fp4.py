@@ -130,6 +130,22 @@ def test_fp4_few_recovery_slices(n, R, S):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("n,R,chunk_words,words", [
+    (16, 12, 28160, 76800),      # three chunks of 152, 76 and 72 pairs of tiles instead of 100
+    (16, 12, 28160, 76802),      # a last pair of two words
+    (16, 12, 25600, 58368),      # three whole waves exactly
+    (500, 240, 28160, 76802),    # either form
+])
+def test_fp4_chunks_of_two_sizes(n, R, chunk_words, words):
+    L = _lib.load()
+    kbytes = ((n + 15) // 16 * 16) * 8
+    one_tile = (128 * kbytes + 1023) // 1024 * 1024
+    scratch = L.par2cuda_tensor_fp4_scratch_bytes(R, n, 1) - one_tile + chunk_words * kbytes
+    assert L.par2cuda_muladd_launches(R, n, words, _lib.METHOD_TENSOR_FP4, scratch) == 1 + 2 * 3
+    got, want = run_fp4(n, R, 2 * words, seed=n + R, accumulate=True, scratch_bytes=scratch)
+    assert np.array_equal(got, want)
+
+
 def test_fp4_forms_agree_with_the_field():
     # every coefficient bit against every word bit: 16 x 16 single-bit products
     import torch
