@@ -282,19 +282,27 @@ __device__ __forceinline__ uint64_t splitmix_mix(uint64_t z) {
 	z ^= z >> 27; z *= 0x94D049BB133111EBull;
 	return z ^ (z >> 31);
 }
-__global__ void k_synth(uint8_t* dst, size_t pitchBytes, unsigned nRows, size_t rowBytes, uint64_t seed, uint64_t first,
-                        uint64_t unitOffset)
+// Two 8-byte units per thread, rows on the grid's second axis: a unit's row and
+// place from one index cost a 64-bit division each, more than its bytes.
+__global__ void __launch_bounds__(256) k_synth(uint8_t* dst, size_t pitchBytes, unsigned nRows, size_t rowBytes, uint64_t seed,
+                                               uint64_t first, uint64_t unitOffset)
 {
-	const size_t units = (rowBytes + 7) / 8;
-	const size_t total = units * nRows;
-	for(size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x; id < total; id += (size_t)gridDim.x * blockDim.x) {
-		size_t row = id / units, u = id % units;
-		uint64_t z = splitmix_mix(seed * 0xD1342543DE82EF95ull + (first + row) * 0x9E3779B97F4A7C15ull + unitOffset + u);
+	const size_t u = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+	if(u * 8 >= rowBytes) return;
+	for(unsigned row = blockIdx.y; row < nRows; row += gridDim.y) {
+		const uint64_t base = seed * 0xD1342543DE82EF95ull + (first + row) * 0x9E3779B97F4A7C15ull + unitOffset + u;
+		const uint64_t z[2] = {splitmix_mix(base), splitmix_mix(base + 1)};
 		uint8_t* p = dst + row * pitchBytes + u * 8;
-		if(u * 8 + 8 <= rowBytes && ((reinterpret_cast<uintptr_t>(p) & 7) == 0)) {
-			*reinterpret_cast<uint64_t*>(p) = z;
-		} else {
-			for(size_t b = 0; b < 8 && u * 8 + b < rowBytes; b++) p[b] = (uint8_t)(z >> (8 * b));
+		if(u * 8 + 16 <= rowBytes && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+			*reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(z[0], z[1]);
+			continue;
+		}
+#pragma unroll
+		for(int h = 0; h < 2; h++, p += 8) {
+			const size_t at = (u + h) * 8;
+			if(at + 8 <= rowBytes && (reinterpret_cast<uintptr_t>(p) & 7) == 0) *reinterpret_cast<uint64_t*>(p) = z[h];
+			else
+				for(size_t b = 0; b < 8 && at + b < rowBytes; b++) p[b] = (uint8_t)(z[h] >> (8 * b));
 		}
 	}
 }
@@ -303,10 +311,9 @@ int synth_fill(void* dst, size_t pitchBytes, unsigned nRows, size_t rowBytes, ui
                uint64_t byteOffset)
 {
 	if(byteOffset % 8) { set_error("synthetic window offset must be a multiple of 8"); return -1; }
-	size_t total = (rowBytes + 7) / 8 * (size_t)nRows;
-	if(!total) return 0;
-	unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 152 * 32);
-	k_synth<<<blocks, 256, 0, st>>>((uint8_t*)dst, pitchBytes, nRows, rowBytes, seed, first, byteOffset / 8);
+	if(!rowBytes || !nRows) return 0;
+	const dim3 grid((unsigned)((rowBytes + 4095) / 4096), std::min(nRows, 65535u));
+	k_synth<<<grid, 256, 0, st>>>((uint8_t*)dst, pitchBytes, nRows, rowBytes, seed, first, byteOffset / 8);
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
 }

@@ -246,6 +246,19 @@ def test_device_checksum_detects_corruption():
     assert flags.tolist() == [1, 1, 1, 1, 0, 1]
 
 
+@pytest.mark.parametrize("n,S,pitch", [(1, 1, 16), (3, 15, 16), (3, 17, 32), (2, 24, 40), (5, 33, 33), (2, 4095, 4096), (2, 4097, 4112),
+                                       (70000, 9, 12)])   # more rows than a grid's second axis holds; rows off 8-byte boundaries
+def test_synthetic_fill_at_its_edges(n, S, pitch):
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    d = torch.full((n * pitch,), 0xA5, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_synth_fill(d.data_ptr(), pitch, n, S, 77, 3, None), "synth")
+    torch.cuda.synchronize()
+    got = d.cpu().numpy().reshape(n, pitch)
+    assert np.array_equal(got[:, :S], synth.slices(77, 3, n, S))
+    assert (got[:, S:] == 0xA5).all()
+
+
 @pytest.mark.parametrize("n,S,batch,pinned", [(1, 2, 0, False), (40, 1000, 8, False), (40, 1000, 8, True), (300, 100000, 64, True)])
 @pytest.mark.filterwarnings("ignore::pytest.PytestUnraisableExceptionWarning")
 def test_completions_come_once_and_in_order(n, S, batch, pinned):
