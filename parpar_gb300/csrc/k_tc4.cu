@@ -655,6 +655,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				if(j >= T4_TR && !__all_sync(0xffffffffu, t4_wait_ab(bar(T4B_IDEMPTY + slot), ((j / T4_TR) - 1) & 1, abortFlag))) return false;
 				if(el) {
 					const uint32_t idAddr = t4_saddr(const_cast<uint32_t*>(tileIds + slot));
+					// subtracted here, not where it is fetched: there the warp would
+					// wait for the counter's round trip (10 x 1 x 1 MiB 110 -> 104 us)
+					ahead -= tileBase;
 					if(ahead >= nAll) ahead = T4_NO_TILE;
 					// stores that complete on each CTA's barrier (a release at
 					// cluster scope would wait ~2000 clocks for the SM's traffic)
@@ -662,13 +665,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					for(uint32_t c = 0; c < 2; c++)
 						asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];"
 						             :: "r"(t4_mapa(idAddr, c)), "r"(ahead), "r"(t4_mapa(bar(T4B_IDFULL + slot), c)) : "memory");
-					if(ahead != T4_NO_TILE) ahead = atomicAdd(tileCounter, 1u) - tileBase;
+					if(ahead != T4_NO_TILE) ahead = atomicAdd(tileCounter, 1u);
 				}
 				__syncwarp();
 				return true;
 			};
 			if(rank == 0) {
-				if(el) ahead = atomicAdd(tileCounter, 1u) - tileBase;
+				if(el) ahead = atomicAdd(tileCounter, 1u);
 				__syncwarp();
 				ok = publish(0);
 			}
