@@ -148,7 +148,9 @@ int rows_cksum(uint16_t* rows, size_t pitchWords, unsigned nRows, const uint32_t
 	// rows have to fill the chip: two CTAs for each that it holds (six: 3.4
 	// against 4.4 TB/s at 300 x 1 MiB)
 	const size_t fill = (size_t)nRows * Sp / (152 * 2 * CK_CTAS * CK_THREADS);
-	const unsigned laneBytes = (unsigned)std::min<size_t>(512, std::max<size_t>(128, fill / 128 * 128));
+	// (and no more CTAs to a row than a grid's second axis holds)
+	const size_t least = Sp / (65535ull * CK_THREADS) / 128 * 128 + 128;
+	const unsigned laneBytes = (unsigned)std::max(least, std::min<size_t>(512, std::max<size_t>(128, fill / 128 * 128)));
 	const size_t ctaBytes = (size_t)CK_THREADS * laneBytes;
 	dim3 grid(nRows, (unsigned)std::max<size_t>(1, (Sp + ctaBytes - 1) / ctaBytes));
 	k_rows_cksum_partial<<<grid, CK_THREADS, 0, st>>>(rows, pitchWords, dLens, (uint32_t)sliceBytes, sliceBytes, laneBytes,
