@@ -200,7 +200,8 @@ int par2cuda_tc4_shape_for(unsigned num_in);
  * No counterpart in the reference. */
 int par2cuda_md5_chain_rate(double* bytes_per_s, void* stream);
 /* The comb CTA shape the next multiply-accumulate with num_rec recovery rows
- * will use (the set_comb_shape setting, else the automatic choice). */
+ * will use (the set_comb_shape setting, else the automatic choice for many
+ * inputs and long rows; a few of either may take a narrower shape). */
 int par2cuda_comb_shape_for(unsigned num_rec);
 /* Measures the current device's three-input LOP3 throughput (ops/s) with a
  * calibration kernel at full occupancy (about 0.1 s): the denominator of the
@@ -271,7 +272,8 @@ int par2cuda_rows_checksum(uint16_t* d_rows, size_t pitch_words, unsigned num_ro
                            size_t slice_bytes, int verify, uint8_t* d_flags, void* d_scratch, void* stream);
 /* IFSC entries (hasher/hasher_base.h:154-176): for each row i, MD5 of its
  * first d_lens[i] bytes zero-padded to slice_bytes, then CRC32 of the same
- * (little-endian), 20 bytes per row into d_ifsc.  One GPU thread per row.
+ * (little-endian), 20 bytes per row into d_ifsc.  One GPU thread per row for
+ * the MD5, one warp for the CRC.
  * d_lens may be NULL (full rows).  pitch_bytes: multiple of 16. */
 int par2cuda_slice_hash(const void* d_rows, size_t pitch_bytes, unsigned num_rows, const uint32_t* d_lens,
                         size_t slice_bytes, uint8_t* d_ifsc, void* stream);

@@ -29,8 +29,8 @@ static size_t default_batch(size_t slice, int method) {
 	// about 512 MiB of staged input per area, 8..512 inputs, multiple of 8;
 	// the 4-bit tensor method wants long K (16 bits per input) per GEMM: its
 	// per-tile set-up and epilogue are amortised over more MMAs, so 4 GiB per
-	// area, up to 4096 inputs (2000 x 2 MiB slices: 65 ms per pass through the
-	// plugin calls against 96 ms with 256-input batches)
+	// area, up to 4096 inputs (2000 x 2 MiB slices: 39 ms per pass through the
+	// plugin calls; with the kernel's earlier form 65, and 96 in batches of 256)
 	const bool tensor4 = method == 5;
 	size_t b = ((tensor4 ? 4096ull : 512ull) << 20) / (slice ? slice : 1);
 	b = std::min<size_t>(b, tensor4 ? 4096 : 512);

@@ -974,34 +974,51 @@ int comb_error_take() {
 static std::atomic<int> g_comb_shape{0};
 int set_comb_shape(int shape) { return g_comb_shape.exchange(shape); }
 
-// Automatic CTA shape from R (measured on 2000 x 1 MiB, 2000 x 2 MiB and
-// 4096 x 256 KiB jobs): above 8 rows the paired-table kernel wins even with
-// padded rows (R = 16: 2.1 T vs 1.8 T word mul-adds/s for the best narrow
-// shape).  Candidates, with their measured rate per row relative to the
-// 72-row block: 72 rows (6 rows x 12 lookup warps, 1.00), 64 rows (8 x 8,
-// 0.97) and 96 rows (8 x 12 with register reallocation, 1.018); the one with
-// the lowest padded-rows / rate wins above 72 rows.  Up to 8 rows a
-// single-warp one-phase CTA builds its own tables.
-int comb_auto_shape(unsigned R) {
+// Automatic CTA shape.  Ratios are times of the other shape over the chosen one's.
+//
+// Up to 8 rows a single-warp one-phase CTA builds its own tables (shape 1), but
+// where its words are two waves of 128-word CTAs at most, too few such warps
+// are in flight: shape 14 (36 rows, 4 words per lane, one table per slot)
+// 1.0 to 1.8 times as fast at 64 KiB rows of 10 to 1000 inputs, 0.95 to 1.35 at
+// 128 KiB.
+//
+// Up to 36 rows shape 14 also beats the paired tables, whose two slots of two
+// tables a few inputs hardly fill: 100 x 10 x 1 MiB 572 -> 447 us, 200 x 20 x
+// 300 000 bytes 251 -> 211; 1.04 to 1.12 at 250 inputs, but 0.95 to 1.05 at 500
+// and 0.80 to 0.93 at 3000, where each row's index bytes weigh more (up to 12
+// rows it holds to 2500 inputs, 1.01 to 1.08).  Past it, from 24 rows, 60-row
+// blocks (shape 22: 3 rows x 20 lookup warps) beat 72-row ones (16: 6 x 12), 1.01 to
+// 1.07, as they do at 37 to 60 rows for up to 512 inputs (1.01 to 1.08; 0.99 to
+// 1.00 at 1500).
+//
+// Above that the cheapest of 72-, 60- and 96-row blocks (28: 8 x 12 with register
+// reallocation) by what a block costs relative to one of 72: 100 rows 1.03 to
+// 1.05 times as fast as the two 64-row blocks taken before, 256 rows 1.03 to 1.06.
+int comb_auto_shape(unsigned R, unsigned nIn, size_t nWords, bool wide) {
+	if(wide) {   // 8-byte loads of the inputs
+		if(R <= 8 && nWords <= 2 * 152 * 128) return 14;
+		if(R > 8 && ((R <= 12 && nIn <= 1536) || (R <= 36 && nIn <= 256))) return 14;
+	}
 	if(R <= 8) return 1;
-	if(R <= 72) return 16;   // one block either way: measured faster than 64-row blocks at R = 16, 32, 64
-	static const struct { int shape; unsigned rows; double rate; } cand[3] = {{16, 72, 1.0}, {18, 64, 0.97}, {28, 96, 1.018}};
+	if(R < 24) return 16;
+	if(R <= 36 || (R <= 60 && nIn <= 512)) return 22;
+	if(R <= 72) return 16;
+	static const struct { int shape; unsigned rows; double cost; } cand[3] = {{16, 72, 1.0}, {22, 60, 0.96}, {28, 96, 1.27}};
 	int best = 16;
 	double bestCost = 1e300;
 	for(const auto& c : cand) {
-		const double cost = (double)((R + c.rows - 1) / c.rows * c.rows) / c.rate;
+		const double cost = (R + c.rows - 1) / c.rows * c.cost;
 		if(cost < bestCost) { bestCost = cost; best = c.shape; }
 	}
 	return best;
 }
 
+// (for many inputs and long rows)
 int comb_shape_for(unsigned R) {
 	const int s = g_comb_shape.load();
-	return s > 0 ? s : comb_auto_shape(R);
+	return s > 0 ? s : comb_auto_shape(R, ~0u, ~(size_t)0, true);
 }
 
-// Chooses the CTA shape from R: full 96-row blocks for large R, fewer warps /
-// rows per warp for small R so that little of a block is wasted.
 int comb_muladd(const uint16_t* in, size_t inPitch, unsigned nIn, const uint4* idx, uint16_t* rec, size_t recPitch,
                 unsigned R, size_t nWords, int accumulate, int shape, cudaStream_t st)
 {
@@ -1011,7 +1028,7 @@ int comb_muladd(const uint16_t* in, size_t inPitch, unsigned nIn, const uint4* i
 		return 0;
 	}
 	if(shape <= 0) shape = g_comb_shape.load();
-	if(shape <= 0) shape = comb_auto_shape(R);
+	if(shape <= 0) shape = comb_auto_shape(R, nIn, nWords, inPitch % 4 == 0 && reinterpret_cast<uintptr_t>(in) % 8 == 0);
 	switch(shape) {
 	case 1: return launch_comb<8, 1>(in, inPitch, nIn, idx, rec, recPitch, R, nWords, accumulate, st);
 	case 2: return launch_comb<8, 4>(in, inPitch, nIn, idx, rec, recPitch, R, nWords, accumulate, st);

@@ -592,7 +592,7 @@ int file_md5(const void* rows, size_t pitchBytes, unsigned nFiles, const uint64_
 	if(!nFiles) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
 	// one thread per file.  filesPerBlock 1 (default): one file per block,
-	// spread over SMs (the fastest chains: 108 MB/s).  32: one warp of files
+	// spread over SMs (the fastest chains: 144 MB/s).  32: one warp of files
 	// per block, ~6 % slower per chain but ceil(nFiles/32) blocks instead of
 	// nFiles, each of which keeps a full-register-file CTA of other work off
 	// its SM while the chains run.  Up to 512: the files of several jobs on

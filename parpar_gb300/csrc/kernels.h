@@ -48,7 +48,7 @@ int comb_batched(const BatchJob* dJobs, unsigned nJobs, unsigned long long total
 // process-wide CTA shape override for the comb kernel (0 = choose from R); returns the previous value
 int set_comb_shape(int shape);
 // shape chosen for R when none is set
-int comb_auto_shape(unsigned R);
+int comb_auto_shape(unsigned R, unsigned nIn, size_t nWords, bool wide);
 int comb_shape_for(unsigned R);  // the shape the next comb call with R rows uses
 // reads and clears the device error flag of the comb kernels (1 = a bounded wait timed out)
 int comb_error_take();

@@ -246,6 +246,39 @@ def test_device_checksum_detects_corruption():
     assert flags.tolist() == [1, 1, 1, 1, 0, 1]
 
 
+@pytest.mark.parametrize("R", [1, 8, 9, 12, 13, 23, 24, 36, 37, 60, 61, 73, 100, 121])
+@pytest.mark.parametrize("n,nw,pad,off", [(10, 2050, 0, 0), (10, 2050, 2, 0), (256, 322, 0, 2), (257, 130, 0, 0), (513, 66, 0, 0),
+                                          (1537, 64, 0, 0), (10, 38914, 0, 0)])
+def test_automatic_comb_shape_matches_the_72_row_one(R, n, nw, pad, off):
+    # each side of the lines between the shapes; rows off 8-byte boundaries by
+    # their pitch (pad) or their start (off)
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(R * 1000 + n)
+    pw = (nw + 63) // 64 * 64 + pad
+    buf = torch.randint(-32768, 32768, (n * pw + off,), generator=g, device="cuda").to(torch.int16)
+    coeff = torch.randint(-32768, 32768, (R, n), generator=g, device="cuda").to(torch.int16)
+    start = torch.randint(-32768, 32768, (R, pw), generator=g, device="cuda").to(torch.int16)
+    sb = L.par2cuda_muladd_scratch_bytes(R, n)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+    got = {}
+    for shape in (0, 16):
+        rec = start.clone()
+        prev = L.par2cuda_set_comb_shape(shape)
+        try:
+            rc = L.par2cuda_muladd(buf.data_ptr() + 2 * off, pw, n, coeff.data_ptr(), rec.data_ptr(), pw, R, nw, 1, _lib.METHOD_COMB,
+                                   scratch.data_ptr(), sb, None)
+        finally:
+            L.par2cuda_set_comb_shape(prev)
+        assert rc == 0, L.par2cuda_last_error()
+        torch.cuda.synchronize()
+        got[shape] = rec
+    assert L.par2cuda_device_error() == 0
+    assert torch.equal(got[0][:, :nw], got[16][:, :nw])
+    # at most the words up to the next multiple of 64 are written besides
+    assert torch.equal(got[0][:, (nw + 63) // 64 * 64:], start[:, (nw + 63) // 64 * 64:])
+
+
 @pytest.mark.parametrize("n,S,pitch", [(1, 1, 16), (3, 15, 16), (3, 17, 32), (2, 24, 40), (5, 33, 33), (2, 4095, 4096), (2, 4097, 4112),
                                        (70000, 9, 12)])   # more rows than a grid's second axis holds; rows off 8-byte boundaries
 def test_synthetic_fill_at_its_edges(n, S, pitch):
