@@ -70,7 +70,7 @@ enum {
 	T4B_QFULL = 0,                       // compact A landed (local)
 	T4B_QEMPTY = T4B_QFULL + T4_MAXS,      // the expander warps have read it (local)
 	T4B_BFULL = T4B_QEMPTY + T4_MAXS,      // B landed (local)
-	T4B_READY = T4B_BFULL + T4_MAXS,     // L: both CTAs' A expanded and B landed (10 arrivals); by B slot
+	T4B_READY = T4B_BFULL + T4_MAXS,     // L: A expanded and B landed in both CTAs (4 + 1 arrivals each); by B slot
 	T4B_EMPTY = T4B_READY + T4_MAXS,       // the stage's MMAs completed (commit, both CTAs); by B slot
 	T4B_TFULL = T4B_EMPTY + T4_MAXS,      // an accumulator holds a finished pass (commit, both CTAs)
 	T4B_TEMPTY = T4B_TFULL + T4_NACC,    // L: both CTAs' epilogues have read it (16 arrivals)
@@ -434,16 +434,39 @@ __device__ __forceinline__ uint32_t t4_mapa(uint32_t a, uint32_t rank) {
 	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
 	return r;
 }
+// Memory order.  What a barrier's signals order, by who gives them:
+//   T4_CTA   threads and copies of its own CTA (QFULL, QEMPTY, BFULL): CTA
+//            scope, the default of arrivals and waits.
+//   T4_PAIR  threads of either CTA, or MMAs that read both CTAs' shared memory
+//            (READY, EMPTY, IDFULL, IDEMPTY): cluster scope.  An arrival is a
+//            release fence and a relaxed arrival, a wait a relaxed wait and an
+//            acquire fence, both restricted to shared memory, which is all that
+//            these signals guard.
+//   T4_TMEM  accumulators of the pair (TFULL, TEMPTY): cluster scope, relaxed;
+//            the tcgen05 fences beside arrival and wait order TMEM.
+// CTA scope would order nothing between the CTAs.  An unrestricted release or
+// acquire at cluster scope waits ~2000 clocks for whatever the SM has in
+// flight: 4096 x 4096 x 256 KiB takes 28.5 ms with the restricted fences, 49.6
+// without the restriction, 100 x 10 x 1 MiB 0.200 and 0.228.
+enum { T4_CTA, T4_PAIR, T4_TMEM };
+__device__ __forceinline__ void t4_acquire_pair() {
+	asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+}
+template<int BY = T4_CTA>
 __device__ __forceinline__ bool t4_try(uint32_t bar, uint32_t parity) {
 	uint32_t ok;
-	asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-	             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+	if(BY != T4_CTA)
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+	else
+		asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+		             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
 	return ok != 0;
 }
-// the same without waiting
-__device__ __forceinline__ uint32_t t4_test(uint32_t bar, uint32_t parity) {
+// a look at a barrier of the pair, without waiting; the acquire fence is the caller's
+__device__ __forceinline__ uint32_t t4_test_pair(uint32_t bar, uint32_t parity) {
 	uint32_t ok;
-	asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+	asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
 	             : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
 	return ok;
 }
@@ -454,9 +477,13 @@ __device__ __forceinline__ bool t4_wait(uint32_t bar, uint32_t parity) {
 }
 // bounded wait that also gives up when another role of the pair has given up
 // (flags in both CTAs' shared memory), so that one failed wait ends the pair quickly
+template<int BY = T4_CTA>
 __device__ __forceinline__ bool t4_wait_ab(uint32_t bar, uint32_t parity, volatile uint32_t* abortFlag) {
 	for(unsigned i = 0; i < T4_WAIT; i++) {
-		if(t4_try(bar, parity)) return true;
+		if(t4_try<BY>(bar, parity)) {
+			if(BY == T4_PAIR) t4_acquire_pair();
+			return true;
+		}
 		if((i & 1023u) == 1023u && *abortFlag) return false;
 	}
 	atomicExch(&g_tc4_error, 1u);
@@ -469,8 +496,9 @@ __device__ __forceinline__ void t4_arrive(uint32_t bar) {
 	asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(bar) : "memory");
 }
 // arrive on a barrier of either CTA (shared::cluster address)
-__device__ __forceinline__ void t4_arrive_cl(uint32_t bar) {
-	asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory");
+__device__ __forceinline__ void t4_arrive_pair(uint32_t bar) {
+	asm volatile("fence.release.sync_restrict::shared::cta.cluster;\n\t"
+	             "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(bar) : "memory");
 }
 __device__ __forceinline__ void t4_cluster_sync() {
 	asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
@@ -555,7 +583,7 @@ __device__ __forceinline__ uint32_t t4_parity2(uint32_t a, uint32_t b) {
 //           publishes them to both CTAs)
 //   warp 1  leader: issues the pair's MMAs
 //   warp 2  compact A copies
-//   warp 3  (other CTA) tells the leader that a stage is in place
+//   warp 3  tells the leader that a stage's B has landed in this CTA
 //   warps 4-15  expand compact A into e2m1 codes (thread: one word)
 //   warps 16-23 read accumulators out (TMEM lane quarter warp % 4, every other
 //           16 columns), keep the tile's recovery words in registers over the
@@ -633,7 +661,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 	// next tile number of the pair (every role but the scheduler reads them in order)
 	auto next_tile = [&](uint32_t j, unsigned& t) -> bool {
 		const unsigned slot = j % T4_TR;
-		if(!t4_wait_ab(bar(T4B_IDFULL + slot), (j / T4_TR) & 1, abortFlag)) return false;
+		if(!t4_wait_ab<T4_PAIR>(bar(T4B_IDFULL + slot), (j / T4_TR) & 1, abortFlag)) return false;
 		t = tileIds[slot];
 		return true;
 	};
@@ -652,7 +680,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			bool ok = true;
 			auto publish = [&](uint32_t j) -> bool {
 				const unsigned slot = j % T4_TR;
-				if(j >= T4_TR && !__all_sync(0xffffffffu, t4_wait_ab(bar(T4B_IDEMPTY + slot), ((j / T4_TR) - 1) & 1, abortFlag))) return false;
+				if(j >= T4_TR && !__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(bar(T4B_IDEMPTY + slot), ((j / T4_TR) - 1) & 1, abortFlag))) return false;
 				if(el) {
 					const uint32_t idAddr = t4_saddr(const_cast<uint32_t*>(tileIds + slot));
 					// subtracted here, not where it is fetched: there the warp would
@@ -679,7 +707,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				unsigned t = T4_NO_TILE;
 				if(el) t4_expect(bar(T4B_IDFULL + j % T4_TR), 4);
 				if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
-				if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+				__syncwarp();
+				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				if(rank == 0 && !publish(j + 1)) break;
 				unsigned mt, nt;
@@ -689,7 +718,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				for(unsigned e = stages; e; e--, g++) {
 					const uint32_t bytes = (left > 1 ? full : tail) * unitBytes;
 					if(--left == 0) left = spr;
-					if(g >= nB && !__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_EMPTY + s), ph, abortFlag))) { ok = false; break; }
+					if(g >= nB && !__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_EMPTY + s), ph, abortFlag))) { ok = false; break; }
 					if(el) t4_bulk(bBase + s * szB, src, bytes, barBase + 8 * (T4B_BFULL + s));
 					src += bytes;
 					if(++s == nB) { s = 0; ph ^= 1; }
@@ -700,7 +729,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			// still in flight land
 			const bool gone = *abortFlag != 0;
 			for(uint32_t h = g > nB ? g - nB : 0; h < g; h++)
-				if(gone || !t4_wait_ab(bar(T4B_EMPTY + h % nB), (h / nB) & 1, abortFlag))
+				if(gone || !t4_wait_ab<T4_PAIR>(bar(T4B_EMPTY + h % nB), (h / nB) & 1, abortFlag))
 					t4_wait(bar(T4B_BFULL + h % nB), (h / nB) & 1);
 		} else if(warp == 1) {
 			if(rank == 0) {
@@ -722,7 +751,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				auto begin_pass = [&]() -> bool {
 					if(kg) return true;
 					if(np < nGrp) { np++; return true; }
-					if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_TEMPTY + grp), phT, abortFlag))) return false;
+					if(!__all_sync(0xffffffffu, t4_wait_ab<T4_TMEM>(barBase + 8 * (T4B_TEMPTY + grp), phT, abortFlag))) return false;
 					asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 					return true;
 				};
@@ -737,14 +766,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				for(uint32_t j = 0; ok; j++) {
 					unsigned t = T4_NO_TILE;
 					if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
-					if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+					__syncwarp();
+					if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 					if(t == T4_NO_TILE) break;
 					if constexpr(!SHORT) {
 						for(int p = 0; p < P && ok; p++) {
 							if(!begin_pass()) { ok = false; break; }
 							uint32_t acc = 0;
 							for(unsigned left = spr; left; left--) {
-								if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
+								if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
 								asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 								const uint64_t ad = aDesc + saOff, bd = bDesc + sbOff;
 								const uint32_t n = left > 1 ? (uint32_t)T4_SU : tail;
@@ -763,7 +793,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					} else {
 						int p = 0;
 						for(unsigned e = stages; e; e--) {
-							if(!seen && !__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
+							if(seen) t4_acquire_pair();
+							else if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
 							asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 							const uint64_t ad = aDesc + saOff, bd = bDesc + sbOff;
 							const uint32_t empty = barBase + 8 * (T4B_EMPTY + sb);
@@ -771,7 +802,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 							sbOff += szB / 16;
 							if(++sb == nB) { sb = 0; sbOff = 0; phB ^= 1; }
 							// a look at the next stage while this one is issued
-							const uint32_t peek = t4_test(barBase + 8 * (T4B_READY + sb), phB);
+							const uint32_t peek = t4_test_pair(barBase + 8 * (T4B_READY + sb), phB);
 #pragma unroll
 							for(uint32_t k = 0; k < pps; k++) {
 								if(p < P) {
@@ -800,7 +831,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			for(uint32_t j = 0; ok; j++) {
 				unsigned t = T4_NO_TILE;
 				if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
-				if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+				__syncwarp();
+				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				unsigned mt, nt;
 				t4_tile(t, mTiles, nTiles, groupM, mt, nt);
@@ -818,24 +850,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			for(uint32_t h = g > nQ ? g - nQ : 0; h < g; h++)
 				t4_wait(bar(T4B_QFULL + h % nQ), (h / nQ) & 1);
 		} else if(warp == 3) {
-			// in the CTA that does not issue: tells the leader that a stage's A
-			// and B are in place here.  Expanders arrive locally, which puts
-			// their shared-memory writes (fenced to the async proxy) before
-			// this warp's remote arrival, and this SM's own tensor core reads
-			// them: remote arrivals by the expanders themselves overtook their
-			// writes now and then.  A release at cluster scope here would wait
-			// for everything the SM has in flight (~2000 clocks a stage).
+			// B is written by copies, which signal their own CTA's barrier: passed
+			// on to the leader, who waits for A and B of both CTAs at one barrier
+			// (READY).  The expanders arrive there themselves: each thread fences
+			// its writes to the async proxy, the warp joins, and one thread
+			// arrives for it, ordered across the pair as described at t4_try.
 			const uint32_t ready = lead(T4B_READY);
 			uint32_t s = 0, ph = 0;
 			bool ok = true;
 			for(uint32_t j = 0; ok; j++) {
 				unsigned t = T4_NO_TILE;
 				if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
-				if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+				__syncwarp();
+				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				for(unsigned e = stages; e; e--) {
 					if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_BFULL + s), ph, abortFlag))) { ok = false; break; }
-					if(el) t4_arrive_cl(ready + 8 * s);
+					if(el) t4_arrive_pair(ready + 8 * s);
 					if(++s == nB) { s = 0; ph ^= 1; }
 				}
 			}
@@ -854,7 +885,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				unsigned t = T4_NO_TILE;
 				if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
 				__syncwarp();
-				if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				uint32_t e = grp >= turn ? grp - turn : grp + T4_EG - turn;
 				turn = (turn + stages) % T4_EG;
@@ -878,7 +909,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					if(qs >= nQ) { qs -= nQ; qph ^= 1; }
 					// the MMAs of the slot's previous stage (NA stages before) have completed
 					if(seq >= nA) {
-						if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_EMPTY + eb), eph, abortFlag))) { ok = false; break; }
+						if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_EMPTY + eb), eph, abortFlag))) { ok = false; break; }
 						eb += T4_EG;
 						if(eb >= nB) { eb -= nB; eph ^= 1; }
 					} else {
@@ -890,7 +921,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					for(int k = 0; k < 3 * T4_SU; k++) if(k < 3 * (int)n) ap[k * 128] = t4_codes_a(q[k]);
 					asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 					__syncwarp();
-					if(el) t4_arrive_cl(ready + 8 * sb);
+					if(el) t4_arrive_pair(ready + 8 * sb);
 					sa += T4_EG;
 					if(sa >= nA) sa -= nA;
 					sb += T4_EG;
@@ -913,7 +944,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			unsigned t = T4_NO_TILE;
 			if(!__all_sync(0xffffffffu, next_tile(j, t))) break;
 			__syncwarp();
-			if(el) t4_arrive_cl(lead(T4B_IDEMPTY + j % T4_TR));
+			if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 			if(t == T4_NO_TILE) break;
 			unsigned mt, nt;
 			t4_tile(t, mTiles, nTiles, groupM, mt, nt);
@@ -923,7 +954,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 #pragma unroll
 				for(int e = 0; e < PAIRS; e++) st[i][e] = 0;
 			for(int p = 0; p < P;) {
-				if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_TFULL + grp), phT, abortFlag))) { ok = false; break; }
+				if(!__all_sync(0xffffffffu, t4_wait_ab<T4_TMEM>(barBase + 8 * (T4B_TFULL + grp), phT, abortFlag))) { ok = false; break; }
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 				const int pEnd = min(P, p + (int)PG);
 				uint32_t col = tq + grp * PG * BN + 16 * half;
@@ -958,7 +989,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				// this warp's TMEM reads are done: the accumulators may take new passes
 				asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 				__syncwarp();
-				if(el) t4_arrive_cl(tempty + 8 * grp);
+				if(el) t4_arrive_pair(tempty + 8 * grp);
 				if(++grp == nGrp) { grp = 0; phT ^= 1; }
 			}
 			if(!ok) break;
