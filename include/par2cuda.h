@@ -279,7 +279,10 @@ int par2cuda_slice_hash(const void* d_rows, size_t pitch_bytes, unsigned num_row
                         size_t slice_bytes, uint8_t* d_ifsc, void* stream);
 /* File MD5s (HasherInput::end, hasher/hasher_base.h:178-186): file f is the
  * d_file_len[f] bytes held by consecutive rows from d_first_row[f], each row
- * holding slice_bytes of it.  One GPU thread per file; 16 bytes per file. */
+ * holding slice_bytes of it.  One GPU thread per file; 16 bytes per file.
+ * pitch_bytes: multiple of 16; d_rows: 16-byte aligned if slice_bytes is a
+ * multiple of 64, else at any address (read by bytes where rows do not begin
+ * at, and consist of, whole 4-byte words). */
 int par2cuda_file_md5(const void* d_rows, size_t pitch_bytes, unsigned num_files, const uint64_t* d_file_len,
                       const uint32_t* d_first_row, size_t slice_bytes, uint8_t* d_md5, void* stream);
 /* par2cuda_file_md5 with 32 files per warp instead of one per block: each

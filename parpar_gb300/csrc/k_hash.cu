@@ -523,6 +523,9 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 	const unsigned f = blockIdx.x * blockDim.x + threadIdx.x;
 	if(f >= nFiles) return;
 	const uint64_t total = fileLen[f];
+	// rows of whole words at 4-byte boundaries (the pitch is a multiple of 16);
+	// any others are read by bytes
+	const bool words = sliceBytes % 4 == 0 && reinterpret_cast<uintptr_t>(rows) % 4 == 0;
 	uint32_t st[4];
 	md5_init(st);
 	uint32_t tail[16];
@@ -540,8 +543,8 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 			const size_t full = take / 64;
 			md5_blocks(st, reinterpret_cast<const uint4*>(p), full);
 			pos = full * 64;
-		} else if((sliceBytes % 4) == 0 && take >= 64) {
-			// rows of whole words: the words that complete the block the last
+		} else if(words && take >= 64) {
+			// the words that complete the block the last
 			// row began, then blocks from a 4-byte boundary; what is left
 			// (whole words but in a file's last row) begins the next block
 			const uint32_t* d32 = reinterpret_cast<const uint32_t*>(p);
@@ -559,10 +562,10 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 			if(MAXT > 32) md5_blocks32(st, d32 + pos / 4, full);
 			else md5_blocks_words(st, d32 + pos / 4, full);
 			pos += full * 64;
-			const uint32_t words = (uint32_t)(take - pos) / 4;
+			const uint32_t left = (uint32_t)(take - pos) / 4;
 #pragma unroll
-			for(uint32_t q = 0; q < 16; q++) if(q < words) tail[q] = __ldg(d32 + pos / 4 + q);
-			tailLen = 4 * words;
+			for(uint32_t q = 0; q < 16; q++) if(q < left) tail[q] = __ldg(d32 + pos / 4 + q);
+			tailLen = 4 * left;
 			pos += tailLen;
 		}
 		for(; pos < take; pos++) {

@@ -223,3 +223,26 @@ def test_ifsc_partial_blocks_of_neighbouring_rows(S):
     for i in range(n):
         padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
         assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4, 13])
+@pytest.mark.parametrize("S", [100, 4100, 72, 33])
+def test_file_md5_of_rows_at_any_address(S, offset):
+    """Slice sizes that are no multiple of a 64-byte block: the rows may begin at any byte."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    lengths = [1, 63, 64, S - 1, S, S + 1, 2 * S + 3, 5 * S + S // 2]
+    files = [synth.slice_bytes(700 + S, k, n) for k, n in enumerate(lengths)]
+    d, pitch, lens, first, nrows = _rows_from_files(torch, files, S)
+    moved = torch.zeros(d.numel() * d.element_size() + 16, dtype=torch.uint8, device="cuda")
+    moved[offset:offset + moved.numel() - 16] = d.view(torch.uint8).reshape(-1)
+    want = b"".join(hashlib.md5(f.tobytes()).digest() for f in files)
+    flen = torch.tensor(lengths, dtype=torch.int64, device="cuda")
+    d_first = torch.from_numpy(first.view(np.int32)).cuda()
+    for call in (L.par2cuda_file_md5, L.par2cuda_file_md5_packed,
+                 lambda *a: L.par2cuda_file_md5_pooled(*a[:7], 64, a[7])):
+        md5 = torch.zeros(16 * len(files), dtype=torch.uint8, device="cuda")
+        _lib.check(call(moved.data_ptr() + offset, pitch, len(files), flen.data_ptr(), d_first.data_ptr(), S, md5.data_ptr(),
+                        None), "file_md5")
+        torch.cuda.synchronize()
+        assert md5.cpu().numpy().tobytes() == want
