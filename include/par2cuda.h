@@ -273,7 +273,7 @@ int par2cuda_rows_checksum(uint16_t* d_rows, size_t pitch_words, unsigned num_ro
 /* IFSC entries (hasher/hasher_base.h:154-176): for each row i, MD5 of its
  * first d_lens[i] bytes zero-padded to slice_bytes, then CRC32 of the same
  * (little-endian), 20 bytes per row into d_ifsc.  One GPU thread per row for
- * the MD5, one warp for the CRC.
+ * the MD5 and one warp for the CRC, or one thread for both (short or many rows).
  * d_lens may be NULL (full rows).  pitch_bytes: multiple of 16. */
 int par2cuda_slice_hash(const void* d_rows, size_t pitch_bytes, unsigned num_rows, const uint32_t* d_lens,
                         size_t slice_bytes, uint8_t* d_ifsc, void* stream);

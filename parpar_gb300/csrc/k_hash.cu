@@ -157,6 +157,36 @@ __device__ __forceinline__ void md5_blocks(uint32_t st[4], const uint4* p4, size
 	md5_blocks_at<0>(st, reinterpret_cast<const uint32_t*>(p4), full);
 }
 
+// The same in two buffers with a copy per block: fewer registers and a shorter
+// loop, for many chains per SM.  CRC: the words go through a CRC32 register too,
+// in the bubbles of the MD5's dependency chain.
+struct CrcTabs;
+__device__ __forceinline__ uint32_t crc_word(const CrcTabs& T, uint32_t crc, uint32_t w);
+template<bool CRC>
+__device__ __forceinline__ void md5_blocks_pairs(uint32_t st[4], uint32_t& crc, const CrcTabs* T, const uint4* p4, size_t full) {
+	const uint32_t* p = reinterpret_cast<const uint32_t*>(p4);
+	uint32_t A[16], B[16];
+	if(full > 0) md5_load<0>(p, 0, false, A);
+	if(full > 1) md5_load<0>(p, 1, false, B);
+	auto block = [&](uint32_t (&X)[16], size_t next) {
+		uint32_t m[16];
+#pragma unroll
+		for(int q = 0; q < 16; q++) m[q] = X[q];
+		if(next < full) md5_load<0>(p, next, false, X);
+		if(CRC) {
+#pragma unroll
+			for(int q = 0; q < 16; q++) crc = crc_word(*T, crc, m[q]);
+		}
+		md5_block(st, m);
+	};
+	for(size_t b = 0; b < full; b += 2) {
+		if(b + P2C_MD5_L2_AHEAD < full)
+			asm volatile("prefetch.global.L2 [%0];" :: "l"(p4 + (b + P2C_MD5_L2_AHEAD) * 4));
+		block(A, b + 2);
+		if(b + 1 < full) block(B, b + 3);
+	}
+}
+
 // The same from any 4-byte boundary with 32-bit loads: fewer registers, for
 // blocks of many warps.
 __device__ __forceinline__ void load_block32(const uint32_t* p, size_t b, uint32_t m[16]) {
@@ -453,11 +483,60 @@ __global__ void __launch_bounds__(P2C_IFSC_THREADS) k_slice_hash(const uint8_t* 
 	}
 }
 
+// The same with one thread per row for both hashes: for short rows, where the
+// CRC blocks' tables and joins cost more than the rows, and for many, where the
+// MD5 chains of eight lanes a warp want more issue slots than there are.
+__global__ void __launch_bounds__(128) k_slice_hash_rows(const uint8_t* rows, size_t pitch, unsigned n, const uint32_t* lens,
+                                                         size_t sliceBytes, uint8_t* out)
+{
+	__shared__ CrcTabs T;
+	crc_tabs_build(T);
+	const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i >= n) return;
+	const size_t len = lens ? min((size_t)lens[i], sliceBytes) : sliceBytes;
+	const uint8_t* p = rows + (size_t)i * pitch;
+	uint32_t st[4];
+	md5_init(st);
+	uint32_t crc = 0xFFFFFFFFu;
+	const size_t full = len / 64;
+	md5_blocks_pairs<true>(st, crc, &T, reinterpret_cast<const uint4*>(p), full);
+	uint32_t tail[16];
+#pragma unroll
+	for(int q = 0; q < 16; q++) tail[q] = 0;
+	const uint32_t rem = (uint32_t)(len - full * 64);
+	for(uint32_t k = 0; k < rem; k++) {
+		const uint32_t byte = p[full * 64 + k];
+		tail[k >> 2] |= byte << (8 * (k & 3));
+		crc = crc_byte(T, crc, byte);
+	}
+	md5_finish(st, tail, rem, sliceBytes - len, sliceBytes);
+	crc = ~crc_zero_extend(crc, sliceBytes - len);
+	uint8_t* o = out + (size_t)i * 20;
+#pragma unroll
+	for(int w = 0; w < 4; w++) {
+		o[4 * w] = (uint8_t)st[w]; o[4 * w + 1] = (uint8_t)(st[w] >> 8);
+		o[4 * w + 2] = (uint8_t)(st[w] >> 16); o[4 * w + 3] = (uint8_t)(st[w] >> 24);
+	}
+	o[16] = (uint8_t)crc; o[17] = (uint8_t)(crc >> 8); o[18] = (uint8_t)(crc >> 16); o[19] = (uint8_t)(crc >> 24);
+}
+
 int slice_hash(const void* rows, size_t pitchBytes, unsigned n, const uint32_t* dLens, size_t sliceBytes,
                uint8_t* dOut, cudaStream_t st)
 {
 	if(!n) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
+	// Rows up to which the split form is as fast or faster (times of the thread
+	// form over the split form's): 1024-byte rows 1.11 at 1000, 0.91 at 2000; 2048
+	// 1.13 at 2000, 0.74 at 4000; 4096 1.07 at 4000, 0.94 at 5000; 8192 1.06 at
+	// 6000, 0.86 at 8000; 16384 1.07 at 8000, 0.94 at 9000; from 32 KiB 1.02 at
+	// 10 000 and 0.91 to 0.95 at 12 000.  Below 1 KiB never: 512 bytes 0.86 to 1.00.
+	const size_t most = sliceBytes < 1024 ? 0 : sliceBytes <= 4096 ? sliceBytes :
+	                    std::min<size_t>(4096 + (sliceBytes - 4096) / 2, sliceBytes >= 32768 ? 10000 : 8192);
+	if(n > most) {
+		k_slice_hash_rows<<<(n + 127) / 128, 128, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dLens, sliceBytes, dOut);
+		P2C_CUDA_TRY(cudaGetLastError());
+		return 0;
+	}
 	const unsigned md5Blocks = (n + P2C_IFSC_ROWS - 1) / P2C_IFSC_ROWS, per = P2C_IFSC_THREADS / 32;
 	k_slice_hash<<<md5Blocks + (n + per - 1) / per, P2C_IFSC_THREADS, 0, st>>>((const uint8_t*)rows, pitchBytes, n, md5Blocks, dLens,
 	                                                                          sliceBytes, dOut);

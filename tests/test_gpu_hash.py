@@ -246,3 +246,23 @@ def test_file_md5_of_rows_at_any_address(S, offset):
                         None), "file_md5")
         torch.cuda.synchronize()
         assert md5.cpu().numpy().tobytes() == want
+
+
+@pytest.mark.parametrize("n,S", [(10, 1020), (1024, 1024), (1025, 1024), (4096, 4096), (4097, 4096), (6144, 8192), (6145, 8192),
+                                 (32768, 68)])
+def test_ifsc_of_short_and_many_rows(n, S):
+    """Both sides of the row counts at which one thread per row takes over, with full, short, empty and odd rows."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    pitch = L.par2cuda_row_pitch_bytes(S)
+    lens = np.array([(S, S - 1, 0, 64 * (i % (S // 64 + 1)), i % (S + 1))[i % 5] for i in range(n)], dtype=np.uint32)
+    rows = synth.slices(82, 0, n, pitch)
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_lens = torch.from_numpy(lens.view(np.int32)).cuda()
+    out = torch.zeros(n * 20, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_slice_hash(d.data_ptr(), pitch, n, d_lens.data_ptr(), S, out.data_ptr(), None), "slice_hash")
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(n, 20)
+    for i in range(n):
+        padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
+        assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
