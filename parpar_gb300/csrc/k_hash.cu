@@ -525,13 +525,18 @@ int slice_hash(const void* rows, size_t pitchBytes, unsigned n, const uint32_t* 
 {
 	if(!n) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
-	// Rows up to which the split form is as fast or faster (times of the thread
-	// form over the split form's): 1024-byte rows 1.11 at 1000, 0.91 at 2000; 2048
-	// 1.13 at 2000, 0.74 at 4000; 4096 1.07 at 4000, 0.94 at 5000; 8192 1.06 at
-	// 6000, 0.86 at 8000; 16384 1.07 at 8000, 0.94 at 9000; from 32 KiB 1.02 at
-	// 10 000 and 0.91 to 0.95 at 12 000.  Below 1 KiB never: 512 bytes 0.86 to 1.00.
-	const size_t most = sliceBytes < 1024 ? 0 : sliceBytes <= 4096 ? sliceBytes :
-	                    std::min<size_t>(4096 + (sliceBytes - 4096) / 2, sliceBytes >= 32768 ? 10000 : 8192);
+	// Rows up to which the split form is the faster one.  The thread form takes
+	// the time of one chain up to 16 000 rows; the split form takes less of it,
+	// until its CRC blocks take more: a row costs them a fixed part, one per 512
+	// bytes and one per byte past those (in the chain's bytes: 680, 42 and 1.3).
+	// Times of the thread form over the split form's: 1024 bytes 1.11 at 1000 rows,
+	// 0.84 at 2000; 1500 1.15 at 500, 0.83 at 1500; 3000 1.28 at 2000, 0.87 at 3000;
+	// 4096 1.07 at 4000, 0.94 at 5000; 6000 1.16 at 3500, 0.95 at 4500; 12000 1.11 at
+	// 6000, 0.92 at 7000; 16384 1.08 at 8000, 0.95 at 8200.  From there on the MD5
+	// warps are too many: 32 KiB 1.19 at 8000, 0.98 at 10 000.  Below 1 KiB the
+	// split form never wins (512 bytes 0.86 to 1.00).
+	const size_t most = sliceBytes < 1024 ? 0 :
+		std::min<size_t>(1000 * sliceBytes / (680 + 42 * (sliceBytes / 512) + 13 * (sliceBytes % 512) / 10), sliceBytes >= 32768 ? 9000 : 8192);
 	if(n > most) {
 		k_slice_hash_rows<<<(n + 127) / 128, 128, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dLens, sliceBytes, dOut);
 		P2C_CUDA_TRY(cudaGetLastError());

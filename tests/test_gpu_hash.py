@@ -248,8 +248,8 @@ def test_file_md5_of_rows_at_any_address(S, offset):
         assert md5.cpu().numpy().tobytes() == want
 
 
-@pytest.mark.parametrize("n,S", [(10, 1020), (1024, 1024), (1025, 1024), (4096, 4096), (4097, 4096), (6144, 8192), (6145, 8192),
-                                 (32768, 68)])
+@pytest.mark.parametrize("n,S", [(10, 1020), (1340, 1024), (1341, 1024), (1085, 1500), (1086, 1500), (4031, 4096), (4032, 4096),
+                                 (8192, 24576), (8193, 24576), (32768, 68)])
 def test_ifsc_of_short_and_many_rows(n, S):
     """Both sides of the row counts at which one thread per row takes over, with full, short, empty and odd rows."""
     torch = pytest.importorskip("torch")
