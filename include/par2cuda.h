@@ -274,7 +274,8 @@ int par2cuda_rows_checksum(uint16_t* d_rows, size_t pitch_words, unsigned num_ro
  * first d_lens[i] bytes zero-padded to slice_bytes, then CRC32 of the same
  * (little-endian), 20 bytes per row into d_ifsc.  One GPU thread per row for
  * the MD5 and one warp for the CRC, or one thread for both (short or many rows).
- * d_lens may be NULL (full rows).  pitch_bytes: multiple of 16. */
+ * d_lens may be NULL (full rows).  pitch_bytes: multiple of 16; d_rows: 16-byte
+ * aligned unless every row holds less than 64 bytes. */
 int par2cuda_slice_hash(const void* d_rows, size_t pitch_bytes, unsigned num_rows, const uint32_t* d_lens,
                         size_t slice_bytes, uint8_t* d_ifsc, void* stream);
 /* File MD5s (HasherInput::end, hasher/hasher_base.h:178-186): file f is the

@@ -537,7 +537,9 @@ int slice_hash(const void* rows, size_t pitchBytes, unsigned n, const uint32_t* 
 	// split form never wins (512 bytes 0.86 to 1.00).
 	const size_t most = sliceBytes < 1024 ? 0 :
 		std::min<size_t>(1000 * sliceBytes / (680 + 42 * (sliceBytes / 512) + 13 * (sliceBytes % 512) / 10), sliceBytes >= 32768 ? 9000 : 8192);
-	if(n > most) {
+	// (and rows that are not 16-byte aligned: the thread form reads rows shorter
+	// than a block by bytes)
+	if(n > most || reinterpret_cast<uintptr_t>(rows) % 16) {
 		k_slice_hash_rows<<<(n + 127) / 128, 128, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dLens, sliceBytes, dOut);
 		P2C_CUDA_TRY(cudaGetLastError());
 		return 0;

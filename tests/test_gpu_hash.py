@@ -266,3 +266,24 @@ def test_ifsc_of_short_and_many_rows(n, S):
     for i in range(n):
         padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
         assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3, 4, 13])
+@pytest.mark.parametrize("S", [4, 33, 63, 2000])
+def test_ifsc_of_short_rows_at_any_address(S, offset):
+    """Rows of less than a block may begin at any byte."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    n, pitch = 35, 64
+    lens = np.array([(S, 0, S - 1, S // 2, i % S)[i % 5] for i in range(n)], dtype=np.uint32) % 64
+    rows = synth.slices(81, 0, n, pitch)
+    d = torch.zeros(n * pitch + 16, dtype=torch.uint8, device="cuda")
+    d[offset:offset + n * pitch] = torch.from_numpy(rows.reshape(-1).copy()).cuda()
+    d_lens = torch.from_numpy(lens.view(np.int32)).cuda()
+    out = torch.zeros(n * 20, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_slice_hash(d.data_ptr() + offset, pitch, n, d_lens.data_ptr(), S, out.data_ptr(), None), "slice_hash")
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().reshape(n, 20)
+    for i in range(n):
+        padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
+        assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
