@@ -878,12 +878,16 @@ int hash_error_take() {
 
 // ---- MD5 of equal-length rows (recovery packets; MD5Multi, hasher/hasher.h:33-56)
 // row i: prefix[i] (prefixLen bytes, host-assembled packet header) followed by
-// dataLen bytes of row data.  One thread per row.
-__global__ void __launch_bounds__(32 * 32 / P2C_MD5_LANES) k_rows_md5(const uint8_t* rows, size_t pitch, unsigned n, size_t dataLen,
+// dataLen bytes of row data.  One thread per row, LANES of a warp; WHOLE: the
+// prefix is whole blocks (or none), so that the rows' blocks are the stream's.
+// (An instantiation each: in one kernel the loops of both get slower code,
+// 65 536 bytes of 1000 rows 0.53 instead of 0.46 ms.)
+template<int LANES, bool WHOLE>
+__global__ void __launch_bounds__(32 * 32 / LANES) k_rows_md5(const uint8_t* rows, size_t pitch, unsigned n, size_t dataLen,
                                                  const uint8_t* prefix, unsigned prefixLen, uint8_t* out)
 {
-	const unsigned lane = threadIdx.x & 31, i = blockIdx.x * 32 + (threadIdx.x >> 5) * P2C_MD5_LANES + lane;
-	if(lane >= P2C_MD5_LANES || i >= n) return;
+	const unsigned lane = threadIdx.x & 31, i = blockIdx.x * 32 + (threadIdx.x >> 5) * LANES + lane;
+	if(lane >= LANES || i >= n) return;
 	uint32_t st[4];
 	md5_init(st);
 	uint32_t tail[16];
@@ -897,8 +901,8 @@ __global__ void __launch_bounds__(32 * 32 / P2C_MD5_LANES) k_rows_md5(const uint
 	}
 	const uint8_t* p = rows + (size_t)i * pitch;
 	size_t pos = 0;
-	if(tailLen == 0) {
-		md5_blocks(st, reinterpret_cast<const uint4*>(p), dataLen / 64);
+	if(WHOLE) {
+		md5_blocks_words(st, reinterpret_cast<const uint32_t*>(p), dataLen / 64);
 		pos = dataLen / 64 * 64;
 	} else if(tailLen % 4 == 0 && dataLen >= 64 - tailLen) {
 		// a prefix of whole words (the 36-byte packet header): complete its
@@ -934,8 +938,18 @@ int rows_md5(const void* rows, size_t pitchBytes, unsigned n, size_t dataLen, co
 	if(!n) return 0;
 	if(pitchBytes % 16) { set_error("row pitch must be a multiple of 16 bytes"); return -1; }
 	// 32 rows per block: a chain's latency is what counts, so the rows are
-	// spread over the SMs
-	k_rows_md5<<<(n + 31) / 32, 32 * 32 / P2C_MD5_LANES, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dataLen, dPrefix, prefixLen, dOut);
+	// spread over the SMs, and a warp has as few chains as leave one warp to a
+	// scheduler: two share it at a loss (prefix of 36 bytes, 65 536 bytes a row,
+	// times at 8, 16 and 32 lanes: 4864 rows 0.50, 0.52, 0.54 ms; 5000 0.55, 0.52, 0.54;
+	// 9728 0.54, 0.51, 0.52; 10 000 0.74, 0.55, 0.53; 32 768 1.61, 1.03, 0.72).
+	const unsigned schedulers = 152 * 4;
+	auto launch = [&](auto kernel, unsigned lanes) {
+		kernel<<<(n + 31) / 32, 32 * 32 / lanes, 0, st>>>((const uint8_t*)rows, pitchBytes, n, dataLen, dPrefix, prefixLen, dOut);
+	};
+	const bool whole = prefixLen % 64 == 0;
+	if(n <= 8 * schedulers) launch(whole ? k_rows_md5<8, true> : k_rows_md5<8, false>, 8);
+	else if(n <= 16 * schedulers) launch(whole ? k_rows_md5<16, true> : k_rows_md5<16, false>, 16);
+	else launch(whole ? k_rows_md5<32, true> : k_rows_md5<32, false>, 32);
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
 }

@@ -287,3 +287,22 @@ def test_ifsc_of_short_rows_at_any_address(S, offset):
     for i in range(n):
         padded = rows[i, :lens[i]].tobytes() + bytes(S - int(lens[i]))
         assert got[i].tobytes() == hashlib.md5(padded).digest() + zlib.crc32(padded).to_bytes(4, "little"), (i, lens[i])
+
+
+@pytest.mark.parametrize("n", [4864, 4865, 9728, 9729, 9800])
+@pytest.mark.parametrize("prefix", [0, 36, 64])
+def test_rows_md5_of_many_rows(n, prefix):
+    """Both sides of the row counts at which a warp takes more rows."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    data, pitch = 200, 256
+    rows = synth.slices(83, 0, n, pitch)
+    pre = synth.slices(84, 0, n, max(prefix, 2))[:, :prefix]
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_pre = torch.from_numpy(np.ascontiguousarray(pre)).cuda() if prefix else None
+    out = torch.zeros(16 * n, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_rows_md5(d.data_ptr(), pitch, n, data, d_pre.data_ptr() if prefix else None, prefix, out.data_ptr(),
+                                   None), "rows_md5")
+    torch.cuda.synchronize()
+    want = b"".join(hashlib.md5(pre[i].tobytes() + rows[i, :data].tobytes()).digest() for i in range(n))
+    assert out.cpu().numpy().tobytes() == want
