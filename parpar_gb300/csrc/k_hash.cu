@@ -600,8 +600,12 @@ int md5_chain_rate(double* bytesPerSec, cudaStream_t st) {
 
 // ---- per-file MD5 -----------------------------------------------------------
 // file f = rows first[f] .. first[f]+ceil(len[f]/sliceBytes)-1, each row
-// contributing sliceBytes bytes except the last.  One thread per file.
-template<int MAXT>
+// contributing sliceBytes bytes except the last.  One thread per file.  MANY:
+// for blocks of many warps, whose chains take turns at the schedulers: loops with
+// fewer registers and instructions, an instantiation each for slices of whole
+// blocks (WHOLE) and others, whose code is slower in one kernel (1000 files of 256 KiB,
+// 64 a block: 2.18 against 2.52 ms; slices of 65 500 bytes 3.43 against 3.78).
+template<int MAXT, bool MANY, bool WHOLE>
 __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t pitch, unsigned nFiles,
                                                    const uint64_t* fileLen, const uint32_t* firstRow,
                                                    size_t sliceBytes, uint8_t* out)
@@ -624,10 +628,12 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 		const size_t take = (size_t)min((uint64_t)sliceBytes, total - done);
 		const uint8_t* p = rows + row * pitch;
 		size_t pos = 0;
-		if((sliceBytes % 64) == 0) {
+		if(MANY ? WHOLE : sliceBytes % 64 == 0) {
 			// every row starts a block
 			const size_t full = take / 64;
-			md5_blocks(st, reinterpret_cast<const uint4*>(p), full);
+			uint32_t none = 0;
+			if(MANY) md5_blocks_pairs<false>(st, none, nullptr, reinterpret_cast<const uint4*>(p), full);
+			else md5_blocks(st, reinterpret_cast<const uint4*>(p), full);
 			pos = full * 64;
 		} else if(words && take >= 64) {
 			// the words that complete the block the last
@@ -645,7 +651,7 @@ __global__ void __launch_bounds__(MAXT) k_file_md5(const uint8_t* rows, size_t p
 				for(int q = 0; q < 16; q++) tail[q] = 0;
 			}
 			const size_t full = (take - pos) / 64;
-			if(MAXT > 32) md5_blocks32(st, d32 + pos / 4, full);
+			if(MANY) md5_blocks32(st, d32 + pos / 4, full);
 			else md5_blocks_words(st, d32 + pos / 4, full);
 			pos += full * 64;
 			const uint32_t left = (uint32_t)(take - pos) / 4;
@@ -688,9 +694,9 @@ int file_md5(const void* rows, size_t pitchBytes, unsigned nFiles, const uint64_
 	// as few SMs as possible (a warp issues one instruction per ~4-cycle
 	// dependency step, so a few warps per scheduler do not slow each other).
 	if(filesPerBlock == 1) {
-		k_file_md5<32><<<nFiles, 1, 0, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow, sliceBytes, dOut);
+		k_file_md5<32, false, false><<<nFiles, 1, 0, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow, sliceBytes, dOut);
 	} else if(filesPerBlock == 32) {
-		k_file_md5<32><<<(nFiles + 31) / 32, 32, 0, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow,
+		k_file_md5<32, false, false><<<(nFiles + 31) / 32, 32, 0, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow,
 		                                                   sliceBytes, dOut);
 	} else {
 		if(filesPerBlock % 32 || filesPerBlock > 512) {
@@ -698,8 +704,8 @@ int file_md5(const void* rows, size_t pitchBytes, unsigned nFiles, const uint64_
 			return -1;
 		}
 		const unsigned per = min(filesPerBlock, (nFiles + 31) / 32 * 32);
-		k_file_md5<512><<<(nFiles + per - 1) / per, per, 0, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
-		                                                             dFirstRow, sliceBytes, dOut);
+		(sliceBytes % 64 ? k_file_md5<512, true, false> : k_file_md5<512, true, true>)<<<(nFiles + per - 1) / per, per, 0, st>>>(
+			(const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow, sliceBytes, dOut);
 	}
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
