@@ -16,10 +16,10 @@
 
 namespace p2c {
 
-// chains per warp of the hash kernels with a block of many rows or files: the
-// loads of 32 chains of a warp are 32 separate lines or rows of banks, and
-// delay each other; one thread hashes 127.6 MB/s among 32 of a warp, 130.5
-// among 16 and 135.0 among 8 (two warps a scheduler for 64 chains)
+// chains per warp of the IFSC's split form: the loads of 32 chains of a warp are
+// 32 separate lines or rows of banks, and delay each other; one thread hashes
+// 127.6 MB/s among 32 of a warp, 130.5 among 16 and 135.0 among 8 (while warps
+// have a scheduler each: the other kernels choose by the number of chains)
 #define P2C_MD5_LANES 8
 
 // RFC 1321 round constants (a constexpr table: indexed by the unrolled step
@@ -740,15 +740,16 @@ __device__ __forceinline__ bool hs_wait(uint32_t bar, uint32_t parity) {
 	return false;
 }
 
-template<int NT>
-__global__ void __launch_bounds__(NT * 32 / P2C_MD5_LANES) k_file_md5_staged(const uint8_t* __restrict__ rows, size_t pitch, unsigned nFiles,
+// NT files per block, LANES of each warp's threads have one.
+template<int NT, int LANES>
+__global__ void __launch_bounds__(NT * 32 / LANES) k_file_md5_staged(const uint8_t* __restrict__ rows, size_t pitch, unsigned nFiles,
                                                         const uint64_t* __restrict__ fileLen,
                                                         const uint32_t* __restrict__ firstRow, size_t sliceBytes,
                                                         uint8_t* __restrict__ out, const uint32_t* __restrict__ outIndex)
 {
 	extern __shared__ __align__(128) uint8_t smem[];
-	const unsigned t = (threadIdx.x >> 5) * P2C_MD5_LANES + (threadIdx.x & 31);
-	const bool mine = (threadIdx.x & 31) < P2C_MD5_LANES;
+	const unsigned t = (threadIdx.x >> 5) * LANES + (threadIdx.x & 31);
+	const bool mine = (threadIdx.x & 31) < LANES;
 	const unsigned f = blockIdx.x * NT + t;
 	uint8_t* ring = smem + (size_t)t * P2C_STG_STRIDE;
 	uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)NT * P2C_STG_STRIDE) + t * P2C_STG_NS;
@@ -862,15 +863,19 @@ int file_md5_staged(const void* rows, size_t pitchBytes, unsigned nFiles, const 
 	if(sliceBytes % 64 || !sliceBytes) { set_error("staged file MD5: slice size must be a multiple of 64 bytes"); return -1; }
 	if(filesPerBlock != 32 && filesPerBlock != 64) { set_error("staged file MD5: 32 or 64 files per block"); return -1; }
 	const size_t smem = (size_t)filesPerBlock * (P2C_STG_STRIDE + 8 * P2C_STG_NS);
-	if(filesPerBlock == 32) {
-		P2C_CUDA_TRY(cudaFuncSetAttribute(k_file_md5_staged<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		k_file_md5_staged<32><<<(nFiles + 31) / 32, 32 * 32 / P2C_MD5_LANES, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
-		                                                             dFirstRow, sliceBytes, dOut, dOutIndex);
-	} else {
-		P2C_CUDA_TRY(cudaFuncSetAttribute(k_file_md5_staged<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-		k_file_md5_staged<64><<<(nFiles + 63) / 64, 64 * 32 / P2C_MD5_LANES, smem, st>>>((const uint8_t*)rows, pitchBytes, nFiles, dFileLen,
-		                                                             dFirstRow, sliceBytes, dOut, dOutIndex);
-	}
+	auto launch = [&](auto kernel, unsigned lanes) -> int {
+		P2C_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+		kernel<<<(nFiles + filesPerBlock - 1) / filesPerBlock, filesPerBlock * 32 / lanes, smem, st>>>(
+			(const uint8_t*)rows, pitchBytes, nFiles, dFileLen, dFirstRow, sliceBytes, dOut, dOutIndex);
+		return 0;
+	};
+	// Four warps an SM, one per scheduler, are the most that do not delay each
+	// other: 8 files a warp in blocks of 32 while every block has an SM to itself,
+	// else 16 (times of 32 files a warp over those of 8 and of 16: 64 files a block 1.03
+	// to 1.00 and 1.07; 32 a block 1.11 and 1.07 up to 4864 files, 0.94 and 1.07 at 5000).
+	const int rc = filesPerBlock == 64 ? launch(k_file_md5_staged<64, 16>, 16)
+	             : nFiles <= 152 * 32 ? launch(k_file_md5_staged<32, 8>, 8) : launch(k_file_md5_staged<32, 16>, 16);
+	if(rc) return rc;
 	P2C_CUDA_TRY(cudaGetLastError());
 	return 0;
 }

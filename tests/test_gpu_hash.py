@@ -306,3 +306,24 @@ def test_rows_md5_of_many_rows(n, prefix):
     torch.cuda.synchronize()
     want = b"".join(hashlib.md5(pre[i].tobytes() + rows[i, :data].tobytes()).digest() for i in range(n))
     assert out.cpu().numpy().tobytes() == want
+
+
+@pytest.mark.parametrize("per", [32, 64])
+@pytest.mark.parametrize("n", [31, 65, 4864, 4865])
+def test_staged_file_md5_of_many_files(n, per):
+    """Both sides of the file count at which a warp takes more files, and part-filled blocks."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    S, pitch = 64, 128
+    lens = np.array([(1, 63, 64, 65, 128, 150)[i % 6] for i in range(n)], dtype=np.int64)
+    first = np.concatenate(([0], np.cumsum((lens + S - 1) // S)[:-1])).astype(np.int32)
+    rows = synth.slices(85, 0, int(first[-1]) + 3, pitch)
+    d = torch.from_numpy(rows.copy()).cuda()
+    d_len, d_first = torch.from_numpy(lens).cuda(), torch.from_numpy(first).cuda()
+    out = torch.zeros(16 * n, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_file_md5_staged(d.data_ptr(), pitch, n, d_len.data_ptr(), d_first.data_ptr(), S, out.data_ptr(), per,
+                                          None), "staged")
+    torch.cuda.synchronize()
+    assert L.par2cuda_device_error() == 0
+    want = b"".join(hashlib.md5(rows[first[i]:first[i] + 3, :S].tobytes()[:lens[i]]).digest() for i in range(n))
+    assert out.cpu().numpy().tobytes() == want
