@@ -29,19 +29,23 @@ namespace p2c {
 // shifts and XORs: four log and antilog look-ups are eight gathers of 32 lines.
 // 2000 x 2 MiB: 1.05 -> 0.64 ms (6.55 TB/s); 300 x 1 MiB 0.097 -> 0.062;
 // 2 x 100 MiB 0.101 -> 0.046; 4000 x 20 000 bytes 0.037 -> 0.033.
+// Rows of up to 8 KiB have CTAs of one warp: the other warps would find little to
+// do and hold registers that more rows could use (32768 x 4 KiB 0.268 -> 0.066 ms,
+// 32768 x 64 bytes 0.113 -> 0.059).
 constexpr unsigned CK_THREADS = 128, CK_CTAS = 5; // CTAs per SM: at 8 (64 registers) the eight loads spill, 5.87 TB/s
-__global__ void __launch_bounds__(CK_THREADS, CK_CTAS) k_rows_cksum_partial(
+template<unsigned THREADS>
+__global__ void __launch_bounds__(THREADS, CK_CTAS * CK_THREADS / THREADS) k_rows_cksum_partial(
 	uint16_t* rows, size_t pitchWords, const uint32_t* lens, uint32_t fixedLen,
 	size_t sliceBytes, unsigned laneBytes, unsigned long long* ckAcc, int zeroTail, GfTables gt)
 {
-	__shared__ uint4 stage[CK_THREADS * 8];
+	__shared__ uint4 stage[THREADS * 8];
 	const unsigned row = blockIdx.x, lane = threadIdx.x & 31;
 	const size_t Sp = round_up_dev(sliceBytes, 8);
 	const size_t end = round_up_dev(Sp, 16);
 	const size_t len = min((size_t)(lens ? lens[row] : fixedLen), Sp);
 	uint8_t* base = reinterpret_cast<uint8_t*>(rows + (size_t)row * pitchWords);
 	uint4* w = stage + (threadIdx.x & ~31u) * 8;
-	const size_t warp0 = ((size_t)blockIdx.y * CK_THREADS + (threadIdx.x & ~31u)) * laneBytes;
+	const size_t warp0 = ((size_t)blockIdx.y * THREADS + (threadIdx.x & ~31u)) * laneBytes;
 	const size_t load0 = warp0 + (size_t)(lane >> 3) * laneBytes + (lane & 7) * 16;
 
 	uint32_t hLo = 0, hHi = 0; // lanes 0-1 and 2-3 of the running Horner value
@@ -146,15 +150,17 @@ int rows_cksum(uint16_t* rows, size_t pitchWords, unsigned nRows, const uint32_t
 	// bytes per lane: the more, the fewer joins (512 against 256: 5.6 and 4.9 TB/s
 	// at 2000 x 2 MiB; 1024 gives no more there and less at 200 rows), but a few
 	// rows have to fill the chip: two CTAs for each that it holds (six: 3.4
-	// against 4.4 TB/s at 300 x 1 MiB)
-	const size_t fill = (size_t)nRows * Sp / (152 * 2 * CK_CTAS * CK_THREADS);
+	// against 4.4 TB/s at 300 x 1 MiB), and a row its CTA
+	const bool warp = Sp <= 32 * 256;
+	const unsigned threads = warp ? 32 : CK_THREADS;
+	const size_t fill = std::min((size_t)nRows * Sp / (152 * 2 * CK_CTAS * CK_THREADS), round_up((Sp + threads - 1) / threads, 128));
 	// (and no more CTAs to a row than a grid's second axis holds)
 	const size_t least = Sp / (65535ull * CK_THREADS) / 128 * 128 + 128;
 	const unsigned laneBytes = (unsigned)std::max(least, std::min<size_t>(512, std::max<size_t>(128, fill / 128 * 128)));
-	const size_t ctaBytes = (size_t)CK_THREADS * laneBytes;
+	const size_t ctaBytes = (size_t)threads * laneBytes;
 	dim3 grid(nRows, (unsigned)std::max<size_t>(1, (Sp + ctaBytes - 1) / ctaBytes));
-	k_rows_cksum_partial<<<grid, CK_THREADS, 0, st>>>(rows, pitchWords, dLens, (uint32_t)sliceBytes, sliceBytes, laneBytes,
-	                                                  dCkAcc, verify ? 0 : 1, gt);
+	(warp ? k_rows_cksum_partial<32> : k_rows_cksum_partial<CK_THREADS>)<<<grid, threads, 0, st>>>(
+		rows, pitchWords, dLens, (uint32_t)sliceBytes, sliceBytes, laneBytes, dCkAcc, verify ? 0 : 1, gt);
 	P2C_CUDA_TRY(cudaGetLastError());
 	k_rows_cksum_finish<<<nRows, 64, 0, st>>>(rows, pitchWords, nRows, sliceBytes, dCkAcc, verify, dFlags);
 	P2C_CUDA_TRY(cudaGetLastError());

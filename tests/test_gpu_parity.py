@@ -351,6 +351,31 @@ def test_device_checksum_at_its_edges(n, S):
     assert flags.tolist() == [1] * n
 
 
+@pytest.mark.parametrize("n,S", [
+    (7000, 5002), (7000, 8190),      # one warp to a row, more than 128 bytes per lane
+    (7000, 8194), (2000, 40_000),    # one CTA
+    (400, 300_012),                  # several
+])
+def test_device_checksum_of_many_rows(n, S):
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    rows, pw = _dev_rows(torch, n, S, S)
+    lens = [(S, S - 1, S // 2 | 1, 0, 15)[i % 5] for i in range(n)]
+    d_lens = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    ck = torch.zeros(n * 8, dtype=torch.uint8, device="cuda")
+    flags = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_rows_checksum(rows.data_ptr(), pw, n, d_lens.data_ptr(), S, 0, None, ck.data_ptr(), None), "ck")
+    _lib.check(L.par2cuda_rows_checksum(rows.data_ptr(), pw, n, None, S, 1, flags.data_ptr(), ck.data_ptr(), None), "verify")
+    torch.cuda.synchronize()
+    Sp = (S + 7) // 8 * 8
+    for i in list(range(0, n, n // 40)) + [n - 1]:
+        host, l = synth.slices(S, i, 1, S)[0], lens[i]
+        got = rows[i].cpu().numpy().view(np.uint8)
+        assert np.array_equal(got[:l], host[:l]) and not got[l:Sp].any() and not got[Sp + 8:].any()
+        assert int.from_bytes(got[Sp:Sp + 8].tobytes(), "little") == O.cksum(host[:l], S)
+    assert flags.tolist() == [1] * n
+
+
 # ------------------------------------------------------------ full-size properties
 def _sampled_check(torch, d_in, pw, n, d_rec, R, S, exps, samples=48, seed=0):
     """rec[r][w] == sum_i c(i, e_r) * in[i][w] at sampled (r, w)."""
