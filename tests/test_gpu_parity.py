@@ -376,6 +376,21 @@ def test_device_checksum_of_many_rows(n, S):
     assert flags.tolist() == [1] * n
 
 
+@pytest.mark.parametrize("S", [1, 8, 16, 18, 33, 64, 1000, 2048, 2050, 4096, 4100])
+@pytest.mark.parametrize("n", [1, 255, 70_000])
+def test_seeded_fill_of_short_rows(n, S):
+    """Several rows to a block, and rows over the grid's second axis."""
+    torch = pytest.importorskip("torch")
+    L = _lib.load()
+    pitch = S + 5 if n < 1000 else (S + 15) // 16 * 16
+    d = torch.full((n, pitch), 0xA5, dtype=torch.uint8, device="cuda")
+    _lib.check(L.par2cuda_synth_fill(d.data_ptr(), pitch, n, S, 5, 11, None), "synth")
+    torch.cuda.synchronize()
+    for i in sorted({0, 1 % n, n // 2, n - 1}):
+        assert np.array_equal(d[i, :S].cpu().numpy(), synth.slices(5, 11 + i, 1, S)[0]), i
+    assert (d[:, S:] == 0xA5).all()
+
+
 # ------------------------------------------------------------ full-size properties
 def _sampled_check(torch, d_in, pw, n, d_rec, R, S, exps, samples=48, seed=0):
     """rec[r][w] == sum_i c(i, e_r) * in[i][w] at sampled (r, w)."""
