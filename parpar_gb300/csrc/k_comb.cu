@@ -28,6 +28,7 @@
 #include "kernels.h"
 
 #include <atomic>
+#include <cmath>
 
 namespace p2c {
 
@@ -976,38 +977,47 @@ int set_comb_shape(int shape) { return g_comb_shape.exchange(shape); }
 
 // Automatic CTA shape.  Ratios are times of the other shape over the chosen one's.
 //
+// A call takes whole waves of CTAs, one to an SM (three of the one-warp shape), and
+// short rows only a few of them, so the shapes are compared by their waves.
+//
 // Up to 8 rows a single-warp one-phase CTA builds its own tables (shape 1), but
 // where its words are two waves of 128-word CTAs at most, too few such warps
 // are in flight: shape 14 (36 rows, 4 words per lane, one table per slot)
 // 1.0 to 1.8 times as fast at 64 KiB rows of 10 to 1000 inputs, 0.95 to 1.35 at
-// 128 KiB.
+// 128 KiB; not where it needs a wave more (20 000 words: 0.67 to 0.81).
 //
 // Up to 36 rows shape 14 also beats the paired tables, whose two slots of two
 // tables a few inputs hardly fill: 100 x 10 x 1 MiB 572 -> 447 us, 200 x 20 x
 // 300 000 bytes 251 -> 211; 1.04 to 1.12 at 250 inputs, but 0.95 to 1.05 at 500
 // and 0.80 to 0.93 at 3000, where each row's index bytes weigh more (up to 12
-// rows it holds to 2500 inputs, 1.01 to 1.08).  Past it, from 24 rows, 60-row
-// blocks (shape 22: 3 rows x 20 lookup warps) beat 72-row ones (16: 6 x 12), 1.01 to
-// 1.07, as they do at 37 to 60 rows for up to 512 inputs (1.01 to 1.08; 0.99 to
-// 1.00 at 1500).
+// rows it holds to 1536 inputs, 1.03; 1.00 at 1600).  One of its waves takes as long as
+// 1.8 of theirs for twice the words (9728 words, one wave either way: 0.60 to 0.80).
+// Past it, from 24 rows, 60-row blocks (shape 22: 3 rows x 20 lookup warps) beat 72-row
+// ones (16: 6 x 12), 1.01 to 1.07, as they do at 37 to 60 rows for up to 512 inputs
+// (1.01 to 1.08; 0.99 to 1.00 at 1500).
 //
-// Above that the cheapest of 72-, 60- and 96-row blocks (28: 8 x 12 with register
-// reallocation) by what a block costs relative to one of 72: 100 rows 1.03 to
-// 1.05 times as fast as the two 64-row blocks taken before, 256 rows 1.03 to 1.06.
+// Above that the cheapest of 72-, 64- (18: 8 x 8), 60- and 96-row blocks (28: 8 x 12
+// with register reallocation) by what a wave of them costs relative to one of 72:
+// 100 rows 1.03 to 1.05 with 60-row blocks over 64-row ones, 256 rows 1.03 to 1.06
+// with 96-row ones in long rows and 0.75 to 0.83 in one to two waves (512 and 4096 words),
+// where 60- or 64-row ones are taken.
 int comb_auto_shape(unsigned R, unsigned nIn, size_t nWords, bool wide) {
+	const double tiles = (double)(nWords / P2C_TILE_WORDS + (nWords % P2C_TILE_WORDS != 0));
+	const auto waves = [](double ctas, double at_once) { return std::ceil(ctas / at_once); };
+	const double wideWaves = waves(std::ceil(tiles / 2), 152);
 	if(wide) {   // 8-byte loads of the inputs
-		if(R <= 8 && nWords <= 2 * 152 * 128) return 14;
-		if(R > 8 && ((R <= 12 && nIn <= 1536) || (R <= 36 && nIn <= 256))) return 14;
+		if(R <= 8 && nWords <= 2 * 152 * 128 && wideWaves <= waves(tiles, 3 * 152)) return 14;
+		if(R > 8 && ((R <= 12 && nIn <= 1536) || (R <= 36 && nIn <= 256)) && 1.8 * wideWaves < waves(tiles, 152)) return 14;
 	}
 	if(R <= 8) return 1;
 	if(R < 24) return 16;
 	if(R <= 36 || (R <= 60 && nIn <= 512)) return 22;
 	if(R <= 72) return 16;
-	static const struct { int shape; unsigned rows; double cost; } cand[3] = {{16, 72, 1.0}, {22, 60, 0.96}, {28, 96, 1.27}};
+	static const struct { int shape; unsigned rows; double cost; } cand[4] = {{16, 72, 1.0}, {18, 64, 0.955}, {22, 60, 0.94}, {28, 96, 1.27}};
 	int best = 16;
 	double bestCost = 1e300;
 	for(const auto& c : cand) {
-		const double cost = (R + c.rows - 1) / c.rows * c.cost;
+		const double cost = waves(tiles * ((R + c.rows - 1) / c.rows), 152) * c.cost;
 		if(cost < bestCost) { bestCost = cost; best = c.shape; }
 	}
 	return best;

@@ -279,6 +279,14 @@ def test_automatic_comb_shape_matches_the_72_row_one(R, n, nw, pad, off):
     assert torch.equal(got[0][:, (nw + 63) // 64 * 64:], start[:, (nw + 63) // 64 * 64:])
 
 
+@pytest.mark.parametrize("R", [1, 8, 9, 36, 100, 121, 256])
+@pytest.mark.parametrize("n,nw,pad,off", [(10, 512, 0, 0), (10, 19456, 0, 0), (10, 19458, 0, 0), (10, 32770, 0, 0), (10, 32770, 2, 0),
+                                          (257, 9728, 0, 0)])
+def test_automatic_comb_shape_by_waves(R, n, nw, pad, off):
+    # each side of whole waves of the shapes' CTAs
+    test_automatic_comb_shape_matches_the_72_row_one(R, n, nw, pad, off)
+
+
 @pytest.mark.parametrize("n,S,pitch", [(1, 1, 16), (3, 15, 16), (3, 17, 32), (2, 24, 40), (5, 33, 33), (2, 4095, 4096), (2, 4097, 4112),
                                        (70000, 9, 12)])   # more rows than a grid's second axis holds; rows off 8-byte boundaries
 def test_synthetic_fill_at_its_edges(n, S, pitch):
