@@ -234,6 +234,21 @@ size_t par2cuda_tensor_fp4_scratch_bytes(unsigned num_rec, unsigned num_in, size
  * mxf4) issued on shared-memory operands (about 0.1 s): the roofline
  * denominator of that method.  No counterpart in the reference. */
 int par2cuda_tensor_fp4_rate(double* macs_per_s, void* stream);
+/* What a PAR2CUDA_METHOD_TENSOR_FP4 call with these arguments runs on a device
+ * of cta_pairs pairs of SMs (0: GB300's 76): the form (4: 4x4 bit matrices, 7
+ * passes, 112 binary multiply-accumulates per word mul-add; 1: single bits, 63
+ * passes and multiply-accumulates), and how it is laid out.  Needs no GPU.
+ * Returns 0, or -1 where the call would be refused.  No counterpart in the
+ * reference. */
+typedef struct {
+	unsigned form, passes, units;            /* units: K = 96 steps of a pass */
+	unsigned columns, column_tiles;          /* per tile; tiles */
+	unsigned stage_units, group_passes;      /* units of a full stage; passes per accumulator group */
+	unsigned slots_a, slots_b, slots_q;      /* of the rings of A, B and compact A */
+	unsigned chunks, big_chunks;             /* word chunks; those of the first size */
+} par2cuda_tensor_fp4_plan_info;
+int par2cuda_tensor_fp4_plan(unsigned num_rec, unsigned num_in, size_t n_words, size_t scratch_bytes, unsigned cta_pairs,
+                             par2cuda_tensor_fp4_plan_info* out);
 /* The number of kernel launches one par2cuda_muladd call with these
  * arguments makes (the tensor_fp4 method: one per word chunk of expanded
  * input planes and GEMM, plus the coefficient expansion).  No counterpart in

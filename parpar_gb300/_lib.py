@@ -49,6 +49,12 @@ class Info(ctypes.Structure):
     ]
 
 
+class Fp4Plan(ctypes.Structure):
+    _fields_ = [(f, ctypes.c_uint) for f in (
+        "form", "passes", "units", "columns", "column_tiles", "stage_units", "group_passes", "slots_a", "slots_b", "slots_q",
+        "chunks", "big_chunks")]
+
+
 # every exported symbol of include/par2cuda.h: (name, restype, argtypes)
 _vp, _sz, _i, _u, _u16, _u64 = ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_uint, ctypes.c_uint16, ctypes.c_uint64
 SIGNATURES = [
@@ -103,6 +109,7 @@ SIGNATURES = [
     ("par2cuda_file_md5_staged_indexed", _i, [_vp, _sz, _u, _vp, _vp, _vp, _sz, _vp, _u, _vp]),
     ("par2cuda_copy_rows", _i, [_vp, _sz, _vp, _sz, _sz, _u, _vp]),
     ("par2cuda_tensor_fp4_scratch_bytes", _sz, [_u, _u, _sz]),
+    ("par2cuda_tensor_fp4_plan", _i, [_u, _u, _sz, _sz, _u, ctypes.POINTER(Fp4Plan)]),
     ("par2cuda_tensor_fp4_rate", _i, [ctypes.POINTER(ctypes.c_double), _vp]),
     ("par2cuda_wait_selftest", _i, [_u, ctypes.POINTER(_i), ctypes.POINTER(ctypes.c_double)]),
     ("par2cuda_rows_md5", _i, [_vp, _sz, _u, _sz, _vp, _u, _vp, _vp]),

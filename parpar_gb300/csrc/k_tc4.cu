@@ -907,7 +907,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					if(el) t4_arrive(barBase + 8 * (T4B_QEMPTY + qs));
 					qs += T4_EG;
 					if(qs >= nQ) { qs -= nQ; qph ^= 1; }
-					// the MMAs of the slot's previous stage (NA stages before) have completed
+					// the MMAs of the slot's previous stage (nA stages before) have
+					// completed.  A group waits for every third stage only, so it
+					// has not waited for this barrier's phase before: that one had
+					// completed when its last wait was over, as the stages complete,
+					// and their commits signal, in the order of issue (nB > 3 stages
+					// back is before its last one, and nB >= nA keeps this phase
+					// the last one completed)
 					if(seq >= nA) {
 						if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_EMPTY + eb), eph, abortFlag))) { ok = false; break; }
 						eb += T4_EG;
@@ -1173,11 +1179,29 @@ static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t 
 	return have;
 }
 
+// what t4_run makes of a plan: passes per accumulator group (at least two groups
+// fit TMEM beside each other), and the rings
+static unsigned t4_group_passes(const T4Plan& pl) { return std::max(1u, std::min(pl.P, (T4_SF_COL / pl.BN) / 2)); }
+static unsigned t4_stage_units(const T4Plan& pl) { return pl.U < T4_SU ? T4_SU / pl.U * pl.U : T4_SU; }
+
 static int t4_pairs_on_device(unsigned* out) {
 	int dev = 0, nSM = 0;
 	P2C_CUDA_TRY(cudaGetDevice(&dev));
 	P2C_CUDA_TRY(cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev));
 	*out = (unsigned)std::max(nSM / 2, 1);
+	return 0;
+}
+
+int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[12]) {
+	T4Plan pl;
+	if(!R || !nWords || !nIn || !nPairsSM || !t4_plan(pl, R, nIn, nWords, scratchBytes, nPairsSM)) {
+		set_error("tensor method (mxf4): no plan for %u x %u x %zu words in %zu bytes of scratch", nIn, R, nWords, scratchBytes);
+		return -1;
+	}
+	const unsigned rings = t4_rings(t4_stage_units(pl), pl.BN);
+	const unsigned v[12] = {(unsigned)pl.form, pl.P, pl.U, pl.BN, pl.nTiles, t4_stage_units(pl), t4_group_passes(pl),
+	                        rings & 15u, rings >> 4 & 15u, rings >> 8 & 15u, pl.chunks, pl.nBig};
+	std::copy(v, v + 12, out);
 	return 0;
 }
 
@@ -1224,9 +1248,7 @@ static int t4_run(const T4Plan& pl, const uint16_t* in, size_t inPitch, unsigned
 	if(g_tc4_group.load() > 0) groupM = (unsigned)g_tc4_group.load();
 	// each launch advances the tile counter by its tiles + pairs (every pair's
 	// last fetch finds no tile)
-	// passes per accumulator group: at least two groups fit TMEM beside each other
-	const unsigned PG = std::max(1u, std::min(pl.P, (T4_SF_COL / pl.BN) / 2));
-	const unsigned rings = t4_rings(isShort ? T4_SU / pl.U * pl.U : T4_SU, pl.BN);
+	const unsigned PG = t4_group_passes(pl), rings = t4_rings(t4_stage_units(pl), pl.BN);
 	if(!rings) { set_error("tensor method (mxf4): no stage layout for %u columns", pl.BN); return -1; }
 	unsigned base = 0;
 	size_t w0 = 0, wEnd;

@@ -49,7 +49,7 @@ int comb_batched(const BatchJob* dJobs, unsigned nJobs, unsigned long long total
 int set_comb_shape(int shape);
 // shape chosen for R when none is set
 int comb_auto_shape(unsigned R, unsigned nIn, size_t nWords, bool wide);
-int comb_shape_for(unsigned R);  // the shape the next comb call with R rows uses
+int comb_shape_for(unsigned R);  // the shape for R rows of many inputs and long rows (or the override)
 // reads and clears the device error flag of the comb kernels (1 = a bounded wait timed out)
 int comb_error_take();
 // measured three-input LOP3 throughput of the current device (ops/s)
@@ -103,6 +103,7 @@ int tc4_error_take();
 int tc4_mma_rate(double* macsPerSec, cudaStream_t st);
 int set_tc4_shape(int shape);
 int set_tc4_group(int groupM);
+int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[12]);
 unsigned tc4_launches(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes);
 int tc4_shape_for(unsigned kBlocks);
 } // namespace p2c
