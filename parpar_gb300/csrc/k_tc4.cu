@@ -56,7 +56,7 @@ namespace p2c {
 #define T4_TR 4                // ring of published tile numbers
 #define T4_NO_TILE 0xFFFFFFFFu
 #define T4_SF_COL 480          // TMEM columns of the scale factors (all 1.0, shared by A and B)
-#define T4_WAIT (1u << 24)
+#define T4_WAIT (1u << 20)     // polls of a wait before it gives up: some 6 us each, so a few seconds
 #define T4_THREADS 768
 #define T4_EG 3                // groups of four expander warps
 #define T4_EXP_WARPS (4 * T4_EG)
