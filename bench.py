@@ -682,19 +682,24 @@ def roofline_gf(mul_adds, muladd_ms, lop3_ops, n_sm, sm_mhz, kname, alg_bytes):
     return out
 
 
-# binary multiply-accumulates per word mul-add of the 4-bit tensor method's
-# single-bit form (7 GF(16) products of 9 bit products each), the form it takes
-# for the workloads reported here (long passes, many recovery slices)
-TC4_MACS_PER_MUL_ADD = 63
+# binary multiply-accumulates per word mul-add of the 4-bit tensor method's two
+# forms: 7 GF(16) products as 4x4 bit matrices, or as 9 bit products each
+TC4_MACS_PER_MUL_ADD = {4: 112, 1: 63}
 
 
-def roofline_tensor(mul_adds, muladd_ms, mma_macs, kname):
+def roofline_tensor(L, N, R, S, muladd_ms, mma_macs, n_sm, kname):
     """Tensor roofline of the block-scaled 4-bit method: the binary
-    multiply-accumulates it needs (63 per word mul-add) against the MMA rate
-    of the same instruction measured on this device (par2cuda_tensor_fp4_rate);
-    the call's time includes its operand-preparation kernels."""
-    flops = mul_adds * 2 * TC4_MACS_PER_MUL_ADD / (muladd_ms / 1e3)
-    return {"bound": "tensor", "kernel": kname, "achieved": flops / 1e12, "peak": 2 * mma_macs / 1e12,
+    multiply-accumulates of the form that the call takes (with the scratch that
+    the resident jobs give it) against the MMA rate of the same instruction
+    measured on this device (par2cuda_tensor_fp4_rate); the call's time includes
+    its operand-preparation kernels."""
+    words = ((S + 7) // 8 * 8 + 8) // 2
+    plan = _lib.Fp4Plan()
+    _lib.check(L.par2cuda_tensor_fp4_plan(R, N, words, L.par2cuda_tensor_fp4_scratch_bytes(R, N, words), n_sm // 2,
+                                          ctypes.byref(plan)), "tensor_fp4_plan")
+    mul_adds = N * R * (S // 2)
+    flops = mul_adds * 2 * TC4_MACS_PER_MUL_ADD[plan.form] / (muladd_ms / 1e3)
+    return {"bound": "tensor", "kernel": kname, "form": plan.form, "achieved": flops / 1e12, "peak": 2 * mma_macs / 1e12,
             "unit": "TFLOP/s", "frac": flops / (2 * mma_macs), "traffic": None,
             "peak_source": "measured: k_tc4_mma_rate, tcgen05.mma cta_group::2 kind::mxf4 M=256 N=240 K=96 back to back on "
                            "shared-memory operands, one CTA pair per two SMs (nominal dense fp4 of the part: 13.5 PFLOP/s)",
@@ -794,15 +799,18 @@ def run_ours(args, cfg, file_lens):
     peaks = measured_peaks()
     sm_mhz = (clocks or {}).get("sm_mhz") or (peaks or {}).get("sm_max_mhz") or 2070.0
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
+    # (the table kernel's name is that of many inputs and long rows, which all workloads here have)
     kname = _lib.comb_kernel_name(L.par2cuda_comb_shape_for(R)) if args.method in ("comb", "auto") else \
         {"xor": "k_xor_planes", "nibble": "k_nibble_muladd", "tensor": "k_tc_muladd",
          "tensor_fp4": "k_tc4_gemm"}[args.method]
     alg_bytes = (N + R) * S  # read every input once, write every recovery once
     hbm_peak = (peaks or {}).get("hbm_gbs", 6800.0)
-    rgf = roofline_gf(mul_adds, muladd_ms, lop3.value, n_sm, sm_mhz, kname, alg_bytes)
-    if args.traffic_bytes:
+    # the tensor methods execute no integer operations that its peak could bound
+    rgf = None if args.method.startswith("tensor") else \
+        roofline_gf(mul_adds, muladd_ms, lop3.value, n_sm, sm_mhz, kname, alg_bytes)
+    if args.traffic_bytes and rgf:
         rgf["traffic"] = args.traffic_bytes
-    rtc = roofline_tensor(mul_adds, muladd_ms, fp4_rate.value, kname) if args.method == "tensor_fp4" else None
+    rtc = roofline_tensor(L, N, R, S, muladd_ms, fp4_rate.value, n_sm, kname) if args.method == "tensor_fp4" else None
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -851,7 +859,7 @@ def run_ours(args, cfg, file_lens):
     # (the contraction in the job stream and the dense workload)
     if rtc is not None:
         line["roofline_tensor"] = rtc
-    line["roofline"] = dict(rtc if rtc is not None else rgf)
+    line["roofline"] = dict(rtc or rgf or line["roofline_hbm"])
     if dense is not None:
         dm = WORKLOADS["dense"]
         d_mul = dm["N"] * dm["R"] * (dm["S"] // 2)
@@ -860,10 +868,11 @@ def run_ours(args, cfg, file_lens):
             dkn[args.dense_method]
         line["dense"] = {"desc": dm["desc"], "method": args.dense_method, "value": dense["value"], "unit": UNIT,
                          "ms_per_step": dense["ms_per_job"], "steps": dense["jobs"], "e2e": dense.get("e2e"),
-                         "roofline_gf": roofline_gf(d_mul, dense["muladd_ms"], lop3.value, n_sm, sm_mhz, dk,
-                                                    (dm["N"] + dm["R"]) * dm["S"])}
+                         "roofline_gf": None if args.dense_method.startswith("tensor") else
+                         roofline_gf(d_mul, dense["muladd_ms"], lop3.value, n_sm, sm_mhz, dk, (dm["N"] + dm["R"]) * dm["S"])}
         if args.dense_method == "tensor_fp4":
-            line["dense"]["roofline_tensor"] = roofline_tensor(d_mul, dense["muladd_ms"], fp4_rate.value, dk)
+            line["dense"]["roofline_tensor"] = roofline_tensor(L, dm["N"], dm["R"], dm["S"], dense["muladd_ms"],
+                                                               fp4_rate.value, n_sm, dk)
     if not args.no_cpu_baseline and world == 1:
         line["cpu_baseline"] = cpu_baseline_run(cfg, file_lens, os.cpu_count() or 1)
     print(json.dumps(line))
