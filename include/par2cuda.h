@@ -246,6 +246,7 @@ typedef struct {
 	unsigned stage_units, group_passes;      /* units of a full stage; passes per accumulator group */
 	unsigned slots_a, slots_b, slots_q;      /* of the rings of A, B and compact A */
 	unsigned chunks, big_chunks;             /* word chunks; those of the first size */
+	unsigned pass_splits;                    /* tiles that share one's passes (4-byte aligned recovery rows) */
 } par2cuda_tensor_fp4_plan_info;
 int par2cuda_tensor_fp4_plan(unsigned num_rec, unsigned num_in, size_t n_words, size_t scratch_bytes, unsigned cta_pairs,
                              par2cuda_tensor_fp4_plan_info* out);

@@ -52,7 +52,7 @@ class Info(ctypes.Structure):
 class Fp4Plan(ctypes.Structure):
     _fields_ = [(f, ctypes.c_uint) for f in (
         "form", "passes", "units", "columns", "column_tiles", "stage_units", "group_passes", "slots_a", "slots_b", "slots_q",
-        "chunks", "big_chunks")]
+        "chunks", "big_chunks", "pass_splits")]
 
 
 # every exported symbol of include/par2cuda.h: (name, restype, argtypes)

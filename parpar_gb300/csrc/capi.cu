@@ -183,9 +183,9 @@ size_t par2cuda_tensor_fp4_scratch_bytes(unsigned num_rec, unsigned num_in, size
 int par2cuda_tensor_fp4_plan(unsigned num_rec, unsigned num_in, size_t n_words, size_t scratch_bytes, unsigned cta_pairs,
                              par2cuda_tensor_fp4_plan_info* out) {
 	if(!out) { p2c::set_error("tensor_fp4_plan: null output"); return -1; }
-	unsigned v[12];
+	unsigned v[13];
 	if(p2c::tc4_plan_info(num_rec, num_in, n_words, scratch_bytes, cta_pairs ? cta_pairs : 76, v)) return -1;
-	*out = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10], v[11]};
+	*out = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], v[10], v[11], v[12]};
 	return 0;
 }
 

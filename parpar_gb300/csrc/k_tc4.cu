@@ -593,11 +593,15 @@ __device__ __forceinline__ uint32_t t4_parity2(uint32_t a, uint32_t b) {
 // UC > 0: passes of UC < T4_SU units, as many whole passes per stage as fit;
 // UC = 0: a pass is one or more stages (the last with its remainder).
 // Passes accumulate beside each other in groups of PG, signalled as one.
-template<int FORM, unsigned UC>
+// SPLIT: the passes of a tile of words and columns are those of S tiles, each of
+// which adds its passes' share to the recovery words with 32-bit atomics, two words
+// at a time.  (An instantiation: with S known only at run time the unsplit calls were
+// 1 to 4 % slower.)
+template<int FORM, unsigned UC, bool SPLIT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4_gemm(
 	const uint8_t* __restrict__ A, const uint8_t* __restrict__ B, uint16_t* __restrict__ rec, size_t recPitch, unsigned R,
-	unsigned U_, unsigned BN, unsigned PG, unsigned rings, unsigned mTiles, unsigned nTiles, unsigned groupM, size_t w0, size_t nWords,
-	int accumulate, unsigned* __restrict__ tileCounter, unsigned tileBase)
+	unsigned U_, unsigned BN, unsigned PG, unsigned rings, unsigned mTiles, unsigned nTiles, unsigned groupM, unsigned S_, size_t w0,
+	size_t nWords, int accumulate, unsigned* __restrict__ tileCounter, unsigned tileBase)
 {
 	constexpr int P = FORM == 4 ? 7 : 63, CPR = FORM == 4 ? 4 : 1;
 	constexpr bool SHORT = UC > 0;
@@ -613,7 +617,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 	uint32_t* tslot = const_cast<uint32_t*>(tileIds) + T4_TR;
 	volatile uint32_t* abortFlag = tslot + 1;
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const unsigned nAll = mTiles * nTiles;
+	const unsigned S = SPLIT ? S_ : 1u;
+	const unsigned nAll = mTiles * nTiles * S;
 	// a tile is a sequence of runs of stages (UC > 0: one run, of whole passes
 	// per stage; else one run per pass); all stages of a run but the last
 	// have `full` units
@@ -621,7 +626,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 	const unsigned units = P * U;
 	const unsigned spr = SHORT ? (P + pps - 1) / pps : (U + T4_SU - 1) / T4_SU;
 	const unsigned full = SHORT ? pps * U : T4_SU, tail = (SHORT ? units : U) - (spr - 1) * full;
-	const unsigned stages = SHORT ? spr : P * spr;
+	// the first pass of a split, and the stages of split `part`
+	auto pass0 = [&](unsigned part) -> unsigned { return part * P / S; };
+	auto stages_of = [&](unsigned part) -> unsigned { return SHORT ? spr : (pass0(part + 1) - pass0(part)) * spr; };
 	const uint32_t szA = full * T4_UNIT_A, szB = full * BN * 24, szQ = full * T4_UNIT_Q;
 	const uint32_t aBase = sbase;
 	const uint32_t nA = rings & 15u, nB = rings >> 4 & 15u, nQ = rings >> 8 & 15u;
@@ -712,10 +719,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				if(t == T4_NO_TILE) break;
 				if(rank == 0 && !publish(j + 1)) break;
 				unsigned mt, nt;
-				t4_tile(t, mTiles, nTiles, groupM, mt, nt);
-				const uint8_t* src = B + ((size_t)nt * 2 + rank) * units * unitBytes;
+				t4_tile(t / S, mTiles, nTiles, groupM, mt, nt);
+				const uint8_t* src = B + (((size_t)nt * 2 + rank) * units + pass0(t % S) * U) * unitBytes;
 				unsigned left = spr;
-				for(unsigned e = stages; e; e--, g++) {
+				for(unsigned e = stages_of(t % S); e; e--, g++) {
 					const uint32_t bytes = (left > 1 ? full : tail) * unitBytes;
 					if(--left == 0) left = spr;
 					if(g >= nB && !__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_EMPTY + s), ph, abortFlag))) { ok = false; break; }
@@ -770,17 +777,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 					if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 					if(t == T4_NO_TILE) break;
 					if constexpr(!SHORT) {
-						for(int p = 0; p < P && ok; p++) {
+						const unsigned n = pass0(t % S + 1) - pass0(t % S);
+						for(unsigned p = 0; p < n && ok; p++) {
 							if(!begin_pass()) { ok = false; break; }
 							uint32_t acc = 0;
 							for(unsigned left = spr; left; left--) {
 								if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
 								asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 								const uint64_t ad = aDesc + saOff, bd = bDesc + sbOff;
-								const uint32_t n = left > 1 ? (uint32_t)T4_SU : tail;
+								const uint32_t nu = left > 1 ? (uint32_t)T4_SU : tail;
 #pragma unroll
 								for(uint32_t u = 0; u < T4_SU; u++) {
-									if(u < n && el) t4_mma(dacc, ad + u * (T4_UNIT_A / 16), bd + u * bUnit, idesc, sf, acc);
+									if(u < nu && el) t4_mma(dacc, ad + u * (T4_UNIT_A / 16), bd + u * bUnit, idesc, sf, acc);
 									acc = 1;
 								}
 								if(el) t4_commit(barBase + 8 * (T4B_EMPTY + sb));
@@ -788,11 +796,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 								sbOff += szB / 16;
 								if(++sb == nB) { sb = 0; sbOff = 0; phB ^= 1; }
 							}
-							if(ok) end_pass(p == P - 1);
+							if(ok) end_pass(p == n - 1);
 						}
 					} else {
 						int p = 0;
-						for(unsigned e = stages; e; e--) {
+						for(unsigned e = spr; e; e--) {
 							if(seen) t4_acquire_pair();
 							else if(!__all_sync(0xffffffffu, t4_wait_ab<T4_PAIR>(barBase + 8 * (T4B_READY + sb), phB, abortFlag))) { ok = false; break; }
 							asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -835,10 +843,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				unsigned mt, nt;
-				t4_tile(t, mTiles, nTiles, groupM, mt, nt);
-				const uint8_t* src = A + ((size_t)mt * 2 + rank) * units * T4_UNIT_Q;
+				t4_tile(t / S, mTiles, nTiles, groupM, mt, nt);
+				const uint8_t* src = A + (((size_t)mt * 2 + rank) * units + pass0(t % S) * U) * T4_UNIT_Q;
 				unsigned left = spr;
-				for(unsigned e = stages; e; e--, g++) {
+				for(unsigned e = stages_of(t % S); e; e--, g++) {
 					const uint32_t bytes = (left > 1 ? full : tail) * T4_UNIT_Q;
 					if(--left == 0) left = spr;
 					if(g >= nQ && !__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_QEMPTY + s), ph, abortFlag))) { ok = false; break; }
@@ -864,7 +872,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				__syncwarp();
 				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
-				for(unsigned e = stages; e; e--) {
+				for(unsigned e = stages_of(t % S); e; e--) {
 					if(!__all_sync(0xffffffffu, t4_wait_ab(barBase + 8 * (T4B_BFULL + s), ph, abortFlag))) { ok = false; break; }
 					if(el) t4_arrive_pair(ready + 8 * s);
 					if(++s == nB) { s = 0; ph ^= 1; }
@@ -888,6 +896,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 				if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 				if(t == T4_NO_TILE) break;
 				uint32_t e = grp >= turn ? grp - turn : grp + T4_EG - turn;
+				const uint32_t stages = stages_of(t % S);
 				turn = (turn + stages) % T4_EG;
 				uint32_t pos = e;                                    // in its run
 				for(; e < stages; e += T4_EG) {
@@ -953,16 +962,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			if(el) t4_arrive_pair(lead(T4B_IDEMPTY + j % T4_TR));
 			if(t == T4_NO_TILE) break;
 			unsigned mt, nt;
-			t4_tile(t, mTiles, nTiles, groupM, mt, nt);
+			t4_tile(t / S, mTiles, nTiles, groupM, mt, nt);
 			uint32_t st[MY][PAIRS];                          // two recovery words each
 #pragma unroll
 			for(int i = 0; i < MY; i++)
 #pragma unroll
 				for(int e = 0; e < PAIRS; e++) st[i][e] = 0;
-			for(int p = 0; p < P;) {
+			const int pLast = (int)pass0(t % S + 1);
+			for(int p = (int)pass0(t % S); p < pLast;) {
 				if(!__all_sync(0xffffffffu, t4_wait_ab<T4_TMEM>(barBase + 8 * (T4B_TFULL + grp), phT, abortFlag))) { ok = false; break; }
 				asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-				const int pEnd = min(P, p + (int)PG);
+				const int pEnd = min(pLast, p + (int)PG);
 				uint32_t col = tq + grp * PG * BN + 16 * half;
 				for(; p < pEnd; p++, col += BN) {
 					if(16 * half >= BN) continue;
@@ -1000,11 +1010,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T4_THREADS, 1) k_tc4
 			}
 			if(!ok) break;
 			const size_t w = w0 + ((size_t)mt * 2 + rank) * T4_ROWS + 32 * quarter + lane;
-			if(w < nWords) {
-				const unsigned r0 = nt * rpt + half * (16 / CPR);
-				uint16_t* d = rec + (size_t)r0 * recPitch + w;
-				// recovery slices of this warp's columns that exist
-				const unsigned rows = min(R - nt * rpt, rpt);
+			// recovery slices of this warp's columns that exist
+			const unsigned r0 = nt * rpt + half * (16 / CPR), rows = min(R - nt * rpt, rpt);
+			uint16_t* d = rec + (size_t)r0 * recPitch + w;
+			if constexpr(SPLIT) {
+				// an even lane adds its word and the next lane's (whose word is past
+				// the row's only if its own is: an even number of words)
+#pragma unroll
+				for(int i = 0; i < MY; i++) {
+					const unsigned rr = (2 * i + half) * (16 / CPR);
+					if(rr >= rows) break;
+#pragma unroll
+					for(int e = 0; e < 2 * PAIRS; e++) {
+						if(rr + e < rows) {
+							const uint32_t v = st[i][e >> 1] >> (16 * (e & 1)) & 0xFFFFu;
+							const uint32_t next = __shfl_down_sync(0xffffffffu, v, 1);
+							if((lane & 1) == 0 && w < nWords) atomicXor(reinterpret_cast<uint32_t*>(d + (size_t)e * recPitch), v | next << 16);
+						}
+					}
+					d += (size_t)(2 * 16 / CPR) * recPitch;
+				}
+			} else if(w < nWords) {
 #pragma unroll
 				for(int i = 0; i < MY; i++) {
 					const unsigned rr = (2 * i + half) * (16 / CPR);
@@ -1070,6 +1096,7 @@ struct T4Plan {
 	size_t bBytes;         // prepared coefficients
 	size_t pairBytes;      // compact A of 256 words
 	unsigned chunks;       // chunks of words, one preparation and one GEMM launch each
+	unsigned splits;       // tiles that share the passes of one
 	unsigned nBig;         // the first nBig hold bigWords, the others restWords, the last what is left
 	size_t bigWords, restWords;
 	bool fits;             // in the scratch
@@ -1104,8 +1131,10 @@ static unsigned t4_chunks(T4Plan& pl, size_t nWords, size_t cw, size_t capPairs,
 	return (unsigned)mixed;
 }
 
-static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t cw, size_t scratchBytes, unsigned nPairsSM) {
+static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t cw, size_t scratchBytes, unsigned nPairsSM,
+                      bool maySplit) {
 	T4Plan pl;
+	pl.splits = 1;
 	const unsigned cpr = form == 4 ? 4 : 1;
 	const unsigned cap = tc4_shape_for(0) == 2 ? 128 : T4_MAXN;
 	pl.form = form;
@@ -1133,7 +1162,18 @@ static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t 
 	const double stages = (pl.U + T4_SU - 1) / T4_SU;
 	const double pass = 1000 + 100 * stages + pl.U * std::max(0.5 * pl.BN, 68.0);
 	const double pairs = (double)((nWords + 2 * T4_ROWS - 1) / (2 * T4_ROWS));
-	pl.cost = waves * pl.P * pass + 6.7 * nIn * (2 + (form == 4 ? 3.5 : 7.9)) * pairs / nPairsSM;
+	double best = waves * pl.P;
+	// Passes split over tiles that keep idle pairs busy: few words, long passes.
+	// Worth the zeroed rows and atomics where a pair is left with two passes at most
+	// and they are 13 units or more (times whole over split: 500 x 30 x 4 KiB 2.1,
+	// 1000 x 16 x 4 KiB 1.35, 3000 x 60 x 4 KiB 2.25, 3000 x 16 x 256 bytes 2.45; 200 inputs 0.90
+	// to 1.18; with two splits 500 to 10 000 x 16 x 16 KiB 0.91 to 1.00).
+	const unsigned splits = (unsigned)std::min<double>(pl.P, nPairsSM / (pairs * pl.nTiles));
+	if(maySplit && form == 4 && pl.U >= 13 && pl.chunks == 1 && splits >= 4) {
+		pl.splits = splits;
+		best = (pl.P + splits - 1) / splits;
+	}
+	pl.cost = best * pass + 6.7 * nIn * (2 + (form == 4 ? 3.5 : 7.9)) * pairs / nPairsSM;
 	return pl;
 }
 
@@ -1161,7 +1201,8 @@ static size_t t4_min_scratch(unsigned R, unsigned nIn) {
 // false: too little scratch.  The number of word chunks is that of expanded
 // planes of 8 bytes per word and (padded) input in the given scratch, the
 // launch count callers are told; t4_chunks lays them out within that number.
-static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM) {
+static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM,
+                    bool maySplit) {
 	if(scratchBytes < t4_min_scratch(R, nIn)) return false;
 	size_t cw = (scratchBytes - T4_HDR_BYTES - t4_bbytes(R, nIn)) / t4_kbytes(nIn) / T4_ROWS * T4_ROWS;
 	cw = std::min(cw, round_up(nWords, T4_ROWS));
@@ -1170,7 +1211,7 @@ static bool t4_plan(T4Plan& pl, unsigned R, unsigned nIn, size_t nWords, size_t 
 	if(even <= cw && (nWords + even - 1) / even == chunks) cw = even;
 	bool have = false;
 	for(int form : {4, 1}) {
-		const T4Plan c = t4_form(form, R, nIn, nWords, cw, scratchBytes, nPairsSM);
+		const T4Plan c = t4_form(form, R, nIn, nWords, cw, scratchBytes, nPairsSM, maySplit);
 		if(form == 1 && c.U < T4_SU) continue;       // its passes are single stages or more
 		if(!c.fits) continue;
 		if(!have || c.cost < pl.cost) pl = c;
@@ -1192,29 +1233,29 @@ static int t4_pairs_on_device(unsigned* out) {
 	return 0;
 }
 
-int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[12]) {
+int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[13]) {
 	T4Plan pl;
-	if(!R || !nWords || !nIn || !nPairsSM || !t4_plan(pl, R, nIn, nWords, scratchBytes, nPairsSM)) {
+	if(!R || !nWords || !nIn || !nPairsSM || !t4_plan(pl, R, nIn, nWords, scratchBytes, nPairsSM, nWords % 2 == 0)) {
 		set_error("tensor method (mxf4): no plan for %u x %u x %zu words in %zu bytes of scratch", nIn, R, nWords, scratchBytes);
 		return -1;
 	}
 	const unsigned rings = t4_rings(t4_stage_units(pl), pl.BN);
-	const unsigned v[12] = {(unsigned)pl.form, pl.P, pl.U, pl.BN, pl.nTiles, t4_stage_units(pl), t4_group_passes(pl),
-	                        rings & 15u, rings >> 4 & 15u, rings >> 8 & 15u, pl.chunks, pl.nBig};
-	std::copy(v, v + 12, out);
+	const unsigned v[13] = {(unsigned)pl.form, pl.P, pl.U, pl.BN, pl.nTiles, t4_stage_units(pl), t4_group_passes(pl),
+	                        rings & 15u, rings >> 4 & 15u, rings >> 8 & 15u, pl.chunks, pl.nBig, pl.splits};
+	std::copy(v, v + 13, out);
 	return 0;
 }
 
 unsigned tc4_launches(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes) {
 	T4Plan pl;
-	if(!R || !nWords || !nIn || !t4_plan(pl, R, nIn, nWords, scratchBytes, 76)) return 0;
+	if(!R || !nWords || !nIn || !t4_plan(pl, R, nIn, nWords, scratchBytes, 76, true)) return 0;
 	return 1 + 2 * pl.chunks;   // coefficients, then per chunk: inputs + GEMM
 }
 
-typedef decltype(&k_tc4_gemm<4, 0>) T4Gemm;
+typedef decltype(&k_tc4_gemm<4, 0, false>) T4Gemm;
 template<int FORM> static T4Gemm t4_short_gemm(unsigned U) {
 	if(FORM != 4) return nullptr;       // form 1 is chosen for long passes only
-	return U == 1 ? k_tc4_gemm<4, 1> : U == 2 ? k_tc4_gemm<4, 2> : U == 3 ? k_tc4_gemm<4, 3> : k_tc4_gemm<4, 4>;
+	return U == 1 ? k_tc4_gemm<4, 1, false> : U == 2 ? k_tc4_gemm<4, 2, false> : U == 3 ? k_tc4_gemm<4, 3, false> : k_tc4_gemm<4, 4, false>;
 }
 
 template<int FORM>
@@ -1227,8 +1268,9 @@ static int t4_run(const T4Plan& pl, const uint16_t* in, size_t inPitch, unsigned
 	// warpgroups gave up: never launched unless the block's own cover the split
 	cudaFuncAttributes fa;
 	const bool isShort = pl.U < T4_SU;
-	auto gemm = k_tc4_gemm<FORM, 0>;
+	T4Gemm gemm = k_tc4_gemm<FORM, 0, false>;
 	if(isShort) gemm = t4_short_gemm<FORM>(pl.U);
+	if constexpr(FORM == 4) if(pl.splits > 1) gemm = k_tc4_gemm<4, 0, true>;
 	P2C_CUDA_TRY(cudaFuncGetAttributes(&fa, gemm));
 	if(fa.numRegs * T4_THREADS < (T4_THREADS - 32 * T4_EPI_WARPS) * T4_REGS_LOW + 32 * T4_EPI_WARPS * T4_REGS_EPI) {
 		set_error("tensor method (mxf4): %d registers a thread do not cover the kernel's split", fa.numRegs);
@@ -1240,6 +1282,7 @@ static int t4_run(const T4Plan& pl, const uint16_t* in, size_t inPitch, unsigned
 	uint8_t* A = B + pl.bBytes;
 	const unsigned slots = pl.nTiles * (pl.BN / CPR);
 	const size_t nB = (size_t)slots * 3 * pl.U;
+	if(pl.splits > 1 && !accumulate) P2C_CUDA_TRY(cudaMemset2DAsync(rec, recPitch * 2, 0, nWords * 2, R, st));
 	k_tc4_prep_coeff<FORM><<<(unsigned)((nB + 255) / 256), 256, 0, st>>>(coeff, R, nIn, slots, pl.BN, pl.U, B, counter);
 	P2C_CUDA_TRY(cudaGetLastError());
 	// pair tiles per raster group: a wave of CTA pairs then reads about as
@@ -1269,13 +1312,13 @@ static int t4_run(const T4Plan& pl, const uint16_t* in, size_t inPitch, unsigned
 		cfg.blockDim = dim3(T4_PREP_THREADS);
 		P2C_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_tc4_prep_in<FORM>, in, inPitch, nIn, wEnd, w0, (unsigned)items, groups,
 		                                reinterpret_cast<uint32_t*>(A), pl.U, (int)(w0 == 0)));
-		const unsigned nAll = mTiles * pl.nTiles;
+		const unsigned nAll = mTiles * pl.nTiles * pl.splits;
 		const unsigned grid = std::min(nAll, nPairsSM);
 		cfg.gridDim = dim3(2 * grid);
 		cfg.blockDim = dim3(T4_THREADS);
 		cfg.dynamicSmemBytes = T4_SMEM;
 		P2C_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm, (const uint8_t*)A, (const uint8_t*)B, rec, recPitch, R, pl.U, pl.BN, PG, rings,
-		                                mTiles, pl.nTiles, groupM, w0, wEnd, accumulate, counter, base));
+		                                mTiles, pl.nTiles, groupM, pl.splits, w0, wEnd, accumulate, counter, base));
 		base += nAll + grid;
 	}
 	return 0;
@@ -1305,8 +1348,10 @@ int tc4_muladd(const uint16_t* in, size_t inPitch, unsigned nIn, const uint16_t*
 	}
 	unsigned nPairsSM = 0;
 	if(t4_pairs_on_device(&nPairsSM)) return -1;
+	// split passes are added by pairs of words: whole 32-bit words of the rows
+	const bool maySplit = reinterpret_cast<uintptr_t>(rec) % 4 == 0 && recPitch % 2 == 0 && nWords % 2 == 0;
 	T4Plan pl;
-	if(!t4_plan(pl, R, nIn, nWords, scratchBytes, nPairsSM)) {
+	if(!t4_plan(pl, R, nIn, nWords, scratchBytes, nPairsSM, maySplit)) {
 		set_error("tensor method (mxf4): no plan fits %zu bytes of scratch", scratchBytes);
 		return -1;
 	}

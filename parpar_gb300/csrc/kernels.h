@@ -103,7 +103,7 @@ int tc4_error_take();
 int tc4_mma_rate(double* macsPerSec, cudaStream_t st);
 int set_tc4_shape(int shape);
 int set_tc4_group(int groupM);
-int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[12]);
+int tc4_plan_info(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes, unsigned nPairsSM, unsigned out[13]);
 unsigned tc4_launches(unsigned R, unsigned nIn, size_t nWords, size_t scratchBytes);
 int tc4_shape_for(unsigned kBlocks);
 } // namespace p2c

@@ -14,11 +14,15 @@ from parpar_gb300 import _lib
 pytestmark = pytest.mark.gpu
 
 
-def form_of(L, n, R, words):
+def plan_of(L, n, R, words):
     plan = _lib.Fp4Plan()
     sb = L.par2cuda_tensor_fp4_scratch_bytes(R, n, words)
     assert L.par2cuda_tensor_fp4_plan(R, n, words, sb, 0, ctypes.byref(plan)) == 0, L.par2cuda_last_error()
-    return plan.form
+    return plan
+
+
+def form_of(L, n, R, words):
+    return plan_of(L, n, R, words).form
 
 
 @pytest.mark.parametrize("n,R,words,form,reps", [
@@ -87,3 +91,40 @@ def test_single_bit_passes_agree_with_the_field():
     want = O.recover_coeffs(x.view(np.uint8), np.full(unit, 2 * x.shape[1]), coeff[:, :unit].copy()).view(np.int16)
     got = d_rec.cpu().numpy()
     assert np.array_equal(got[:, :x.shape[1]], want) and not got[:, x.shape[1]:].any()
+
+
+@pytest.mark.parametrize("n,R,words,splits", [
+    (289, 1, 2, 7), (300, 7, 130, 7), (500, 30, 2052, 7),    # one tile and several, a last one of two words
+    (1000, 60, 256 * 10, 7), (1000, 61, 256 * 9, 4),         # one column tile and two
+    (3000, 33, 256 * 19, 4), (3000, 33, 256 * 19 + 2, 1),    # both sides of the line
+    (500, 30, 2051, 1),                                      # an odd number of words
+])
+@pytest.mark.parametrize("acc", [0, 1])
+@pytest.mark.parametrize("off", [0, 1])
+def test_split_passes_match_the_table_kernel(n, R, words, splits, acc, off):
+    # off: recovery rows off 4-byte boundaries (never split)
+    import torch
+    L = _lib.load()
+    assert plan_of(L, n, R, words).pass_splits == splits
+    g = torch.Generator(device="cuda").manual_seed(n + words)
+    pw = (words + 63) // 64 * 64
+    d_in, start, d_coeff = (torch.randint(-32768, 32768, shape, generator=g, device="cuda").to(torch.int16)
+                            for shape in ((n, pw), (R, pw), (R, n)))
+    got = {}
+    for method in (_lib.METHOD_COMB, _lib.METHOD_TENSOR_FP4):
+        at = off if method == _lib.METHOD_TENSOR_FP4 else 0
+        buf = torch.full((R * pw + 2,), 0x5A5A, dtype=torch.int16, device="cuda")
+        rec = buf[at:at + R * pw].view(R, pw)
+        rec.copy_(start)
+        sb = L.par2cuda_muladd_scratch_bytes(R, n) if method == _lib.METHOD_COMB else \
+            L.par2cuda_tensor_fp4_scratch_bytes(R, n, words)
+        scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+        assert L.par2cuda_muladd(d_in.data_ptr(), pw, n, d_coeff.data_ptr(), rec.data_ptr(), pw, R, words, acc, method,
+                                 scratch.data_ptr(), sb, None) == 0, L.par2cuda_last_error()
+        torch.cuda.synchronize()
+        got[method] = rec
+        assert buf[R * pw + at:].eq(0x5A5A).all() and buf[:at].eq(0x5A5A).all()
+    assert L.par2cuda_device_error() == 0
+    assert torch.equal(got[_lib.METHOD_COMB][:, :words], got[_lib.METHOD_TENSOR_FP4][:, :words])
+    # nothing past the words was written
+    assert torch.equal(got[_lib.METHOD_TENSOR_FP4][:, words:], start[:, words:])

@@ -97,11 +97,21 @@ class Bar:
 
 
 class Layout:
-    """passes: of a tile; spr: stages of a run; pps: whole passes of a stage (0: a pass is a run of stages)."""
+    """passes: of a tile's words and columns; spr: stages of a run; pps: whole passes of a stage (0: a pass is a
+    run of stages); splits: tiles that share the passes."""
 
-    def __init__(self, nA, nB, nQ, passes, spr, pps, PG, nGrp):
-        self.nA, self.nB, self.nQ, self.passes, self.spr, self.pps, self.PG, self.nGrp = nA, nB, nQ, passes, spr, pps, PG, nGrp
-        self.stages = -(-passes // pps) if pps else passes * spr
+    def __init__(self, nA, nB, nQ, passes, spr, pps, PG, nGrp, splits=1):
+        self.nA, self.nB, self.nQ, self.spr, self.pps, self.PG, self.nGrp = nA, nB, nQ, spr, pps, PG, nGrp
+        self.all_passes, self.splits = passes, splits
+
+    def span(self, t):
+        """First pass of tile t, and the first that is not its own."""
+        part = t % self.splits
+        return part * self.all_passes // self.splits, (part + 1) * self.all_passes // self.splits
+
+    def stages_of(self, t):
+        n = self.span(t)[1] - self.span(t)[0]
+        return -(-n // self.pps) if self.pps else n * self.spr
 
 
 def wait(bar, parity):
@@ -177,7 +187,7 @@ class Pair:
                 yield from publish(j + 1, ahead)
                 if ahead >= 0:
                     ahead = fetch()
-            for _ in range(L.stages):
+            for _ in range(L.stages_of(t)):
                 s = g % L.nB
                 if g >= L.nB:
                     yield from wait(self.empty[r][s], (g // L.nB - 1) & 1)
@@ -200,7 +210,7 @@ class Pair:
             t = yield from self.next_tile(r, j)
             if t < 0:
                 break
-            for _ in range(L.stages):
+            for _ in range(L.stages_of(t)):
                 s = g % L.nQ
                 if g >= L.nQ:
                     yield from wait(self.qempty[r][s], (g // L.nQ - 1) & 1)
@@ -223,7 +233,7 @@ class Pair:
             t = yield from self.next_tile(r, j)
             if t < 0:
                 return
-            for _ in range(L.stages):
+            for _ in range(L.stages_of(t)):
                 yield from wait(self.bfull[r][s], ph)
                 self.ready[s].arrive()
                 s += 1
@@ -240,8 +250,9 @@ class Pair:
             if t < 0:
                 return
             e = grp - turn if grp >= turn else grp + EG - turn
-            turn = (turn + L.stages) % EG
-            while e < L.stages:
+            stages = L.stages_of(t)
+            turn = (turn + stages) % EG
+            while e < stages:
                 stage = base + e
                 yield from wait(self.qfull[r][qs], qph)
                 for _ in range(2):                   # the read takes a while
@@ -270,7 +281,7 @@ class Pair:
                 if sb >= L.nB:
                     sb -= L.nB
                 yield True
-            base += L.stages
+            base += stages
             j += 1
 
     def mma(self):
@@ -288,8 +299,8 @@ class Pair:
             t = yield from self.next_tile(0, j)
             if t < 0:
                 return
-            p = 0
-            for e in range(L.stages):
+            p, last = L.span(t)
+            for e in range(L.stages_of(t)):
                 if not seen:
                     yield from wait(self.ready[sb], ph_b)
                 seen = False
@@ -300,7 +311,7 @@ class Pair:
                 if L.pps:
                     peek = self.ready[sb].passed(ph_b)
                 for k in range(L.pps or 1):
-                    if p >= L.passes:
+                    if p >= last:
                         break
                     if kg == 0 and (L.pps or e % L.spr == 0):
                         if np_ < L.nGrp:
@@ -311,7 +322,7 @@ class Pair:
                     if L.pps or e % L.spr == L.spr - 1:
                         p += 1
                         kg += 1
-                        if kg == L.PG or p == L.passes:
+                        if kg == L.PG or p == last:
                             self.queue.append(lambda gr=grp: [self.tfull[c][gr].arrive() for c in range(2)])
                             kg, grp = 0, grp + 1
                             if grp == L.nGrp:
@@ -329,10 +340,10 @@ class Pair:
             t = yield from self.next_tile(r, j)
             if t < 0:
                 return
-            p = 0
-            while p < L.passes:
+            p, last = L.span(t)
+            while p < last:
                 yield from wait(self.tfull[r][grp], ph)
-                for k in range(min(L.PG, L.passes - p)):
+                for k in range(min(L.PG, last - p)):
                     assert self.acc[grp][k] == (t, p), ("accumulator", self.acc[grp][k], t, p)
                     p += 1
                     yield True
@@ -417,6 +428,36 @@ def test_pair_protocol():
         for seed in range(2):
             rng = random.Random(100 * k + seed)
             run(Layout(*key), rng.randint(1, 6), rng.randint(1, 2), rng)
+
+
+def test_pair_protocol_of_split_passes():
+    # tiles of one to four passes, of unlike lengths, one after another
+    for k, key in enumerate(sorted(key for key in layouts() if not key[5])):
+        for splits in (2, 3, 4, 5, 7):
+            rng = random.Random(1000 * k + splits)
+            run(Layout(*key, splits), splits * rng.randint(1, 3), rng.randint(1, 2), rng)
+
+
+def test_passes_are_split_only_where_pairs_would_idle():
+    lib = _lib.load()
+
+    def splits(n, R, words, pairs=76):
+        plan = _lib.Fp4Plan()
+        sb = lib.par2cuda_tensor_fp4_scratch_bytes(R, n, words)
+        assert lib.par2cuda_tensor_fp4_plan(R, n, words, sb, pairs, ctypes.byref(plan)) == 0
+        assert plan.pass_splits == 1 or (plan.form == 4 and plan.units >= 13 and plan.chunks == 1)
+        return plan.pass_splits
+
+    assert splits(10000, 60, 2052) == 7              # 9 tiles
+    assert splits(10000, 60, 2053) == 1              # an odd number of words
+    assert splits(288, 60, 2052) == 1 and splits(289, 60, 2052) == 7    # 12 units and 13
+    assert splits(3000, 30, 256 * 10) == 7 and splits(3000, 30, 256 * 19) == 4 and splits(3000, 30, 256 * 20) == 1
+    assert splits(3000, 61, 256 * 9) == 4 and splits(3000, 61, 256 * 10) == 1    # two column tiles
+    assert splits(2000, 200, 1 << 20) == 1 and splits(777, 133, 700006) == 1
+    for n in (120, 500, 4096):
+        for R in (1, 60, 61, 300):
+            for words in (2, 256, 4096, 19456, 40000, 200000):
+                splits(n, R, words)
 
 
 def test_pair_protocol_of_63_passes():
