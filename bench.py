@@ -693,6 +693,7 @@ def roofline_tensor(L, N, R, S, muladd_ms, mma_macs, n_sm, kname):
     the resident jobs give it) against the MMA rate of the same instruction
     measured on this device (par2cuda_tensor_fp4_rate); the call's time includes
     its operand-preparation kernels."""
+    from parpar_gb300 import _lib
     words = ((S + 7) // 8 * 8 + 8) // 2
     plan = _lib.Fp4Plan()
     _lib.check(L.par2cuda_tensor_fp4_plan(R, N, words, L.par2cuda_tensor_fp4_scratch_bytes(R, N, words), n_sm // 2,
