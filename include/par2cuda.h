@@ -223,11 +223,13 @@ int par2cuda_wait_selftest(unsigned polls, int* gave_up, double* seconds);
 /* Scratch bytes par2cuda_muladd needs for (num_rec, num_in). */
 size_t par2cuda_muladd_scratch_bytes(unsigned num_rec, unsigned num_in);
 /* Scratch bytes par2cuda_muladd needs for method PAR2CUDA_METHOD_TENSOR_FP4:
- * a 1 KiB header (the GEMM's tile counter, reset by every call), the
- * coefficient bit matrix (16 * roundup(num_rec, 48) rows of
- * roundup(num_in, 16) * 8 bytes) and the 4-bit input planes of a chunk of at
- * most 1 GiB of words (less scratch = smaller chunks; at least one 128-word
- * tile).  No counterpart in the reference. */
+ * a 1 KiB header (the GEMM's tile counter, reset by every call), 16 *
+ * roundup(num_rec, 48) * roundup(num_in, 16) * 8 bytes that hold the prepared
+ * coefficients, and 8 bytes per input (rounded up to 16) and word for the
+ * compact input planes of a chunk of words, at most 1 GiB of them (less scratch
+ * = smaller chunks; at least one 128-word tile).  The planes themselves take
+ * 3.5 or 7.9 bytes, the coefficients 56 or 32 each.  No counterpart in the
+ * reference. */
 size_t par2cuda_tensor_fp4_scratch_bytes(unsigned num_rec, unsigned num_in, size_t n_words);
 /* Measures the tensor pipe's rate (binary multiply-accumulates per second)
  * for the MMA of PAR2CUDA_METHOD_TENSOR_FP4 (a CTA pair's M=256, N=240, K=96,
@@ -251,9 +253,10 @@ typedef struct {
 int par2cuda_tensor_fp4_plan(unsigned num_rec, unsigned num_in, size_t n_words, size_t scratch_bytes, unsigned cta_pairs,
                              par2cuda_tensor_fp4_plan_info* out);
 /* The number of kernel launches one par2cuda_muladd call with these
- * arguments makes (the tensor_fp4 method: one per word chunk of expanded
- * input planes and GEMM, plus the coefficient expansion).  No counterpart in
- * the reference. */
+ * arguments makes (the tensor_fp4 method: the coefficients' preparation, then
+ * the inputs' and a GEMM per word chunk; where it splits passes it also zeroes
+ * the recovery rows with a memset on the stream).  No counterpart in the
+ * reference. */
 int par2cuda_muladd_launches(unsigned num_rec, unsigned num_in, size_t n_words, int method, size_t scratch_bytes);
 /* rec[r][0..n_words) (^)= sum_i coeff[r*num_in + i] * in[i][0..n_words),
  * the run_kernel body (gf16/controller_cpu.cpp:488-515).  Pitches are in

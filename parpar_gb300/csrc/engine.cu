@@ -470,8 +470,9 @@ void Engine::give_event(cudaEvent_t e) {
 // and thrown away): 300 inputs of 1 MiB and 30 outputs took 19.3 ms that way,
 // of which the copies are 2.9.  So completions go out in groups where the host
 // asks for it: those that have completed by the time that this thread looks
-// again, never one held back for work that has not run.  5.1 ms so, and
-// 16 inputs of 64 KiB with 4 outputs 0.51 instead of 1.19.
+// again, never one held back for work that has not run.  5.1 to 6.4 ms so (the
+// host's part varies from run to run), and 16 inputs of 64 KiB with 4 outputs 0.51
+// instead of 1.19.
 void Engine::notify_loop() {
 	cudaSetDevice(device);
 	std::vector<void*> users;

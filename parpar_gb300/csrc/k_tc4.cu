@@ -1108,7 +1108,8 @@ struct T4Plan {
 // wave: 2000 x 200 x 2 MiB, 16 chunks of 3.4 waves cost 64.  Where two sizes,
 // one of whole waves and one above it, come to fewer waves for as many chunks,
 // they are taken (58 there: 11.39 -> 10.66 ms; 4096 x 4096 x 256 KiB, 125 -> 122
-// waves, 28.08 -> 27.63; 4096 x 240 x 256 KiB 3.05 -> 2.77).
+// waves, 28.08 -> 27.63; 4096 x 240 x 256 KiB 3.05 -> 2.77; 1 to 3 % more on either
+// side since the pair's signals have cluster scope).
 static unsigned t4_chunks(T4Plan& pl, size_t nWords, size_t cw, size_t capPairs, unsigned nPairsSM) {
 	const size_t pairWords = 2 * T4_ROWS;
 	auto waves = [&](size_t pairs) { return (pairs * pl.nTiles + nPairsSM - 1) / nPairsSM; };
@@ -1155,8 +1156,10 @@ static T4Plan t4_form(int form, unsigned R, unsigned nIn, size_t nWords, size_t 
 	// a launch takes whole waves of the grid; preparing an input word moves
 	// 2 + 3.5 (form 4) or 2 + 7.9 bytes at 6.7 clocks of the grid per byte
 	// and pair tile.  Form 1 wins where the passes are long and the columns
-	// fill its tiles (ms, form 1 against form 4): 4096 x 4096 x 256 KiB 27.6
-	// and 43.6, 2000 x 200 x 2 MiB 10.7 and 12.1, 1000 x 480 x 1 MiB 5.7 and
+	// fill its tiles (ms, form 1 against form 4): 4096 x 4096 x 256 KiB 28.5
+	// and 45.2, 2000 x 200 x 2 MiB 10.8 and 12.4, 777 x 133 x 1400012 bytes 3.3 and
+	// 2.8, 1000 x 100 x 1 MiB 3.1 and 2.0; before the pair's signals had cluster
+	// scope (1 to 3 % more since, on either side) 1000 x 480 x 1 MiB 5.7 and
 	// 6.0; form 4 for 1000 x 300 x 1 MiB 5.4 and 3.9, 2000 x 100 x 2 MiB 10.1
 	// and 7.2, 500 x 480 x 1 MiB 4.4 and 3.6.
 	const double stages = (pl.U + T4_SU - 1) / T4_SU;
