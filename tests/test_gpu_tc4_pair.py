@@ -128,3 +128,35 @@ def test_split_passes_match_the_table_kernel(n, R, words, splits, acc, off):
     assert torch.equal(got[_lib.METHOD_COMB][:, :words], got[_lib.METHOD_TENSOR_FP4][:, :words])
     # nothing past the words was written
     assert torch.equal(got[_lib.METHOD_TENSOR_FP4][:, words:], start[:, words:])
+
+
+@pytest.mark.parametrize("acc", [0, 1])
+def test_split_passes_in_a_captured_graph(acc):
+    import torch
+    L = _lib.load()
+    n, R, words = 500, 30, 2052
+    assert plan_of(L, n, R, words).pass_splits == 7
+    g = torch.Generator(device="cuda").manual_seed(3)
+    pw = (words + 63) // 64 * 64
+    d_in, start, d_coeff = (torch.randint(-32768, 32768, shape, generator=g, device="cuda").to(torch.int16)
+                            for shape in ((n, pw), (R, pw), (R, n)))
+    rec = start.clone()
+    sb = L.par2cuda_tensor_fp4_scratch_bytes(R, n, words)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+
+    def call(out):
+        assert L.par2cuda_muladd(d_in.data_ptr(), pw, n, d_coeff.data_ptr(), out.data_ptr(), pw, R, words, acc,
+                                 _lib.METHOD_TENSOR_FP4, scratch.data_ptr(), sb,
+                                 torch.cuda.current_stream().cuda_stream) == 0, L.par2cuda_last_error()
+
+    want = start.clone()
+    call(want)                                   # also loads the kernels before the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(rec)
+    for _ in range(3):
+        rec.copy_(start)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(rec, want)
+    assert L.par2cuda_device_error() == 0
